@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/particles_gb300.h"
+#include "pt_detmath.h"
 #include "pt_smul.h"
 
 /* Everything a particle-integration kernel reads, by value in the launch. */
@@ -127,6 +128,29 @@ __host__ __device__ inline PtCarry pt_carry_view(unsigned char *base, int64_t np
 #define PT_REC_FLOATS 11
 #define PT_REC_HEADER_FLOATS 4
 
+/* A double whose +, - and * are separately rounded operations issued as FMAs
+ * (pt_fadd, pt_fsub, pt_fmul): the exact build's expressions keep the
+ * reference's operand order and bits at the FMA rate of the FP64 pipe.  The
+ * other builds write PtR too, as a plain double that contracts. */
+#ifdef PT_EXACT
+struct PtR {
+    double v;
+    __device__ __forceinline__ PtR() {}
+    __device__ __forceinline__ PtR(double x) : v(x) {}
+    __device__ __forceinline__ operator double() const { return v; }
+};
+#define PT_R_OP(op, fn)                                                                              \
+    __device__ __forceinline__ PtR operator op(PtR a, PtR b) { return PtR(fn(a.v, b.v)); }           \
+    __device__ __forceinline__ PtR operator op(PtR a, double b) { return PtR(fn(a.v, b)); }          \
+    __device__ __forceinline__ PtR operator op(double a, PtR b) { return PtR(fn(a, b.v)); }
+PT_R_OP(+, pt_fadd)
+PT_R_OP(-, pt_fsub)
+PT_R_OP(*, pt_fmul)
+#undef PT_R_OP
+#else
+using PtR = double;
+#endif
+
 /* Fortran MIN/MAX with the NaN rule of the oracle (a NaN first operand
  * propagates), and maxval with NaN propagation. */
 __device__ __forceinline__ double pt_max(double a, double b) { return (b > a) ? b : a; }
@@ -190,7 +214,7 @@ __device__ __forceinline__ int32_t pt_node_index(double q, int32_t d)
  * exponent tests run on the integer pipe). */
 __device__ __forceinline__ double pt_qdiv(double a, double b, double y)
 {
-    const double q0 = a * y;
+    const double q0 = pt_fmul(a, y);
     const uint32_t e = (uint32_t)((unsigned long long)__double_as_longlong(q0) >> 52) & 0x7ffu;
     const uint32_t ea = (uint32_t)((unsigned long long)__double_as_longlong(a) >> 52) & 0x7ffu;
     if (e - 63u > 1920u || ea < 116u) return a / b;

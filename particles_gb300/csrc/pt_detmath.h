@@ -22,9 +22,9 @@
  *   - pow(x, y) = exp(y * ln x) for x > 0, with the IEEE special cases that
  *     the step controller can meet (0^negative = +inf, x^0 = 1).
  *
- * Every multiply/add goes through pt_dmul/pt_dadd, which are __dmul_rn /
- * __dadd_rn on the device (never contracted into FMA, whatever -fmad says)
- * and plain operators on the host (the host side must be compiled with
+ * Every multiply/add goes through pt_dmul/pt_dadd, which round once each on
+ * the device (never contracted with one another, whatever -fmad says)
+ * and are plain operators on the host (the host side must be compiled with
  * -ffp-contract=off).  Error bound: (2 + 2|y ln x|) ulp against libm, since
  * z = y ln x is rounded once before exp (tests check it); for the
  * controller's exponents and error ratios that is a few ulp.  Bit-identity
@@ -42,10 +42,30 @@
 #define PT_DM_FN static inline
 #endif
 
+/* On the device a product and a sum are each one fused multiply-add with an
+ * exact neutral operand, a b + (-0) and a 1 + b: one rounding of the same
+ * value, so the same bits (signed zeros included).  GB300's FP64 pipe takes
+ * an FMA of three registers every 64 cycles per scheduler, but DADD, DMUL,
+ * DSETP and an FMA with a constant or immediate operand every 76 (measured
+ * with 4 or more warps per SM).  So the neutral operands must live in
+ * registers: they are formed from %ctaid.z, which is 0 in every launch (the
+ * grids have one z layer) but not known to the compiler. */
+#if defined(__CUDACC__)
+__device__ __forceinline__ double pt_neutral(uint32_t hi)
+{
+    uint32_t z;
+    asm("mov.u32 %0, %%ctaid.z;" : "=r"(z));
+    return __hiloint2double((int)(hi + z), (int)z);
+}
+__device__ __forceinline__ double pt_fmul(double a, double b) { return __fma_rn(a, b, pt_neutral(0x80000000u)); }
+__device__ __forceinline__ double pt_fadd(double a, double b) { return __fma_rn(a, pt_neutral(0x3ff00000u), b); }
+__device__ __forceinline__ double pt_fsub(double a, double b) { return __fma_rn(-b, pt_neutral(0x3ff00000u), a); }
+#endif
+
 PT_DM_FN double pt_dmul(double a, double b)
 {
 #if defined(__CUDA_ARCH__)
-    return __dmul_rn(a, b);
+    return pt_fmul(a, b);
 #else
     return a * b;
 #endif
@@ -54,7 +74,7 @@ PT_DM_FN double pt_dmul(double a, double b)
 PT_DM_FN double pt_dadd(double a, double b)
 {
 #if defined(__CUDA_ARCH__)
-    return __dadd_rn(a, b);
+    return pt_fadd(a, b);
 #else
     return a + b;
 #endif
@@ -63,7 +83,7 @@ PT_DM_FN double pt_dadd(double a, double b)
 PT_DM_FN double pt_dsub(double a, double b)
 {
 #if defined(__CUDA_ARCH__)
-    return __dsub_rn(a, b);
+    return pt_fsub(a, b);
 #else
     return a - b;
 #endif

@@ -49,11 +49,6 @@
 #ifndef PT_SMUL_W
 #define PT_SMUL_W 1
 #endif
-/* Exact build: the force's products on the integer pipes (rolled loop).
- * Off: measured on GB300 it costs 0.7 % on top of the weights' +2.7 %. */
-#ifndef PT_SMUL_FORCE
-#define PT_SMUL_FORCE 0
-#endif
 #define PT_CAT2(a, b) a##_##b
 #define PT_CAT(a, b) PT_CAT2(a, b)
 #define PT_NAME(x) PT_CAT(x, PT_SFX)
@@ -98,16 +93,16 @@ struct EvalF64 {
     {
         constexpr int NV = (NC == 10) ? 9 : 6;
         int32_t l[3], r[3];
-        double xd[3], xu[3];
+        PtR xd[3], xu[3];
 #ifdef PT_EXACT
 #pragma unroll
         for (int i = 0; i < 3; ++i) {                            /* :140-149 */
-            const double x = P.unit_map ? s[i] : pt_qdiv(s[i] - P.xl[i], P.xs[i], P.inv_xs[i]);
-            const double xr = x + P.inv_dm[i];
-            double xp = P.dmr[i] * (xr - pt_floor(xr));
+            const PtR x = P.unit_map ? s[i] : pt_qdiv(pt_fsub(s[i], P.xl[i]), P.xs[i], P.inv_xs[i]);
+            const PtR xr = x + P.inv_dm[i];
+            PtR xp = P.dmr[i] * (xr - pt_floor(xr));
             r[i] = pt_node_index(pt_floor(xp), P.dm[i]);
             xp = P.dmr[i] * (x - pt_floor(x));
-            const double pl = pt_floor(xp);
+            const PtR pl = pt_floor(xp);
             l[i] = pt_node_index(pl, P.dm[i]);
             xd[i] = xp - pl;
             xu[i] = 1.0 - xd[i];
@@ -138,8 +133,8 @@ struct EvalF64 {
         }
 #endif
         /* weights c(1:8) of :207-210; (a*b)*c shares the first product */
-        const double puu = xu[0] * xu[1], pud = xu[0] * xd[1];
-        const double pdu = xd[0] * xu[1], pdd = xd[0] * xd[1];
+        const PtR puu = xu[0] * xu[1], pud = xu[0] * xd[1];
+        const PtR pdu = xd[0] * xu[1], pdd = xd[0] * xd[1];
 #ifndef PT_EXACT
         const double w8[8] = { puu * xu[2], puu * xd[2], pud * xu[2], pud * xd[2],
                                pdu * xu[2], pdu * xd[2], pdd * xu[2], pdd * xd[2] };
@@ -148,7 +143,7 @@ struct EvalF64 {
         const int64_t yl = d1 * l[1], yr = d1 * r[1], zl = d12 * l[2], zr = d12 * r[2];
         const int64_t node[8] = { l[0] + yl + zl, l[0] + yl + zr, l[0] + yr + zl, l[0] + yr + zr,
                                   r[0] + yl + zl, r[0] + yl + zr, r[0] + yr + zl, r[0] + yr + zr };
-        double acc[NV];
+        PtR acc[NV];
         if (P.near) {                          /* interpolate_near (:76-80): the node l */
             double v[NC];
             load_rec<NC>(P.fld, PT_CHK(P, node[0], P.nrec), v);
@@ -170,33 +165,33 @@ struct EvalF64 {
                 return ((q & 4) ? (int64_t)r[0] : (int64_t)l[0]) + ((q & 2) ? yr : yl) + ((q & 1) ? zr : zl);
             };
             auto w_of = [&](int q, bool sw) {
-                const double pxy = (q & 4) ? ((q & 2) ? pdd : pdu) : ((q & 2) ? pud : puu);
-                const double pz = (q & 1) ? xd[2] : xu[2];
-                return sw ? pt_smul_raw(pxy, pz, ok) : pxy * pz;
+                const PtR pxy = (q & 4) ? ((q & 2) ? pdd : pdu) : ((q & 2) ? pud : puu);
+                const PtR pz = (q & 1) ? xd[2] : xu[2];
+                return sw ? PtR(pt_smul_raw(pxy, pz, ok)) : pxy * pz;
             };
             double v[NC], vn[NC];
             load_rec<NC>(P.fld, PT_CHK(P, node[0], P.nrec), v);
             load_rec<NC>(P.fld, PT_CHK(P, node[1], P.nrec), vn);
-            const double wq0 = w_of(0, PT_SMUL_W != 0);
+            const PtR wq0 = w_of(0, PT_SMUL_W != 0);
 #pragma unroll
             for (int cc = 0; cc < NV; ++cc)
-                acc[cc] = cc < PT_SMUL_SPLIT ? pt_smul_raw(wq0, v[cc], ok) : wq0 * v[cc];
+                acc[cc] = cc < PT_SMUL_SPLIT ? PtR(pt_smul_raw(wq0, v[cc], ok)) : wq0 * v[cc];
 #pragma unroll 1
             for (int q = 1; q < 8; ++q) {                         /* :212-220 in order */
 #pragma unroll
                 for (int c = 0; c < NC; ++c) v[c] = vn[c];
                 load_rec<NC>(P.fld, PT_CHK(P, node_of(q < 7 ? q + 1 : 7), P.nrec), vn);
-                const double w = w_of(q, PT_SMUL_W != 0);
+                const PtR w = w_of(q, PT_SMUL_W != 0);
 #pragma unroll
                 for (int cc = 0; cc < NV; ++cc)
-                    acc[cc] = acc[cc] + (cc < PT_SMUL_SPLIT ? pt_smul_raw(w, v[cc], ok) : w * v[cc]);
+                    acc[cc] = acc[cc] + (cc < PT_SMUL_SPLIT ? PtR(pt_smul_raw(w, v[cc], ok)) : w * v[cc]);
             }
             if (!ok) {
 #pragma unroll 1
                 for (int q = 0; q < 8; ++q) {
                     double u[NC];
                     load_rec<NC>(P.fld, PT_CHK(P, node_of(q), P.nrec), u);
-                    const double w = w_of(q, false);
+                    const PtR w = w_of(q, false);
 #pragma unroll
                     for (int cc = 0; cc < NV; ++cc) acc[cc] = (q == 0) ? w * u[cc] : acc[cc] + w * u[cc];
                 }
@@ -214,9 +209,10 @@ struct EvalF64 {
 #ifdef PT_EXACT
         /* the quotients by g and vun through one correctly rounded
          * reciprocal each: bit-identical to the divisions (pt_qdiv) */
-        const double g = sqrt(s[3] * s[3] + s[4] * s[4] + s[5] * s[5] + 1.0);
+        const PtR u0 = s[3], u1 = s[4], u2 = s[5];
+        const double g = sqrt(u0 * u0 + u1 * u1 + u2 * u2 + 1.0);
         const double yg = 1.0 / g;
-        const double v0 = pt_qdiv(s[3], g, yg), v1 = pt_qdiv(s[4], g, yg), v2 = pt_qdiv(s[5], g, yg);
+        const PtR v0 = pt_qdiv(s[3], g, yg), v1 = pt_qdiv(s[4], g, yg), v2 = pt_qdiv(s[5], g, yg);
         a[0] = pt_qdiv(v0, P.vun, P.inv_vun);
         a[1] = pt_qdiv(v1, P.vun, P.inv_vun);
         a[2] = pt_qdiv(v2, P.vun, P.inv_vun);
@@ -228,34 +224,7 @@ struct EvalF64 {
         a[1] = v1 * P.inv_vun;
         a[2] = v2 * P.inv_vun;
 #endif
-        const double w0 = v0 - acc[0], w1 = v1 - acc[1], w2 = v2 - acc[2];
-#if defined(PT_EXACT) && PT_SMUL_FORCE
-        /* The three components in a rolled loop, their products on the
-         * integer pipes (pt_smul_raw), the same expressions as below: a
-         * product outside the integer path's domain clears `okf` and the
-         * FPU form below runs instead. */
-        bool okf = true;
-        double f3 = 0.0, f4 = 0.0, f5 = 0.0;
-#pragma unroll 1
-        for (int c = 0; c < 3; ++c) {
-            const double wa = c == 0 ? w1 : (c == 1 ? w2 : w0);
-            const double ba = c == 0 ? acc[5] : (c == 1 ? acc[3] : acc[4]);
-            const double wb = c == 0 ? w2 : (c == 1 ? w0 : w1);
-            const double bb = c == 0 ? acc[4] : (c == 1 ? acc[5] : acc[3]);
-            double t = pt_smul_raw(wa, ba, okf) - pt_smul_raw(wb, bb, okf);
-            if (NC == 10)
-                t = t + P.eta * (c == 0 ? acc[6 % NV] : (c == 1 ? acc[7 % NV] : acc[8 % NV]));
-            const double val = pt_smul_raw(P.qom, t, okf);
-            f3 = c == 0 ? val : f3;
-            f4 = c == 1 ? val : f4;
-            f5 = c == 2 ? val : f5;
-        }
-        if (okf) {
-            a[3] = f3;
-            a[4] = f4;
-            a[5] = f5;
-        } else
-#endif
+        const PtR w0 = v0 - acc[0], w1 = v1 - acc[1], w2 = v2 - acc[2];
         if (NC == 10) {                                           /* resistive extension */
             a[3] = P.qom * ((w1 * acc[5] - w2 * acc[4]) + P.eta * acc[6 % NV]);
             a[4] = P.qom * ((w2 * acc[3] - w0 * acc[5]) + P.eta * acc[7 % NV]);

@@ -49,11 +49,6 @@
 #ifndef PT_SMUL_STAGE
 #define PT_SMUL_STAGE 1
 #endif
-/* ... and the product by the step size there.  Off: measured on GB300 it
- * costs 1.5 % (six more unrolled integer sequences in the stage slot). */
-#ifndef PT_SMUL_DT
-#define PT_SMUL_DT 0
-#endif
 
 namespace pt_sm {
 
@@ -282,9 +277,9 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
     if (METHOD == PT_METHOD_DOP853) {
         const Stage &S = kDop[j];
         if (j == 1) {                                           /* :368 */
-            const double h = dt * S.a[0];
+            const PtR h = PtR(dt) * S.a[0];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) { dl[c] = h * K(0, c); ss[c] = si[c] + dl[c]; }
+            for (int c = 0; c < 6; ++c) { const PtR d = h * K(0, c); dl[c] = d; ss[c] = si[c] + d; }
         } else {                                                /* :371-415 */
 #if defined(PT_EXACT) && PT_SMUL_STAGE
             /* the coefficient products on the integer pipes (pt_smul_raw:
@@ -293,19 +288,21 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
             bool ok = true;
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                double acc = pt_smul_raw(S.a[0], K(S.r[0], c), ok);
+                PtR acc = pt_smul_raw(S.a[0], K(S.r[0], c), ok);
                 for (int i = 1; i < S.n; ++i) acc = acc + pt_smul_raw(S.a[i], K(S.r[i], c), ok);
-                dl[c] = PT_SMUL_DT ? pt_smul_raw(dt, acc, ok) : dt * acc;
-                ss[c] = si[c] + dl[c];
+                const PtR d = dt * acc;
+                dl[c] = d;
+                ss[c] = si[c] + d;
             }
             if (!ok)
 #endif
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                double acc = S.a[0] * K(S.r[0], c);
-                for (int i = 1; i < S.n; ++i) acc = acc + S.a[i] * K(S.r[i], c);
-                dl[c] = dt * acc;
-                ss[c] = si[c] + dl[c];
+                PtR acc = PtR(S.a[0]) * K(S.r[0], c);
+                for (int i = 1; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i], c);
+                const PtR d = dt * acc;
+                dl[c] = d;
+                ss[c] = si[c] + d;
             }
         }
     } else {                                                    /* :132-135 */
@@ -318,16 +315,16 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
                 dl[c] = acc;
                 ss[c] = si[c] + acc;
             } else {
-                double acc = si[c];
+                PtR acc = si[c];
 #if defined(PT_EXACT) && PT_SMUL_STAGE
                 bool ok = true;
                 for (int i = 0; i < S.n; ++i) acc = acc + pt_smul_raw(S.a[i], K(S.r[i], c), ok);
                 if (!ok) {
                     acc = si[c];
-                    for (int i = 0; i < S.n; ++i) acc = acc + S.a[i] * K(S.r[i], c);
+                    for (int i = 0; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i], c);
                 }
 #else
-                for (int i = 0; i < S.n; ++i) acc = acc + S.a[i] * K(S.r[i], c);
+                for (int i = 0; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i], c);
 #endif
                 ss[c] = acc;
             }
@@ -381,12 +378,13 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
         double sr[6];
 #pragma unroll
         for (int c = 0; c < 6; ++c) {                           /* :418-421, :425 */
-            const double k4 = B01 * K(0, c) + B06 * K(5, c) + B07 * K(6, c) + B08 * K(7, c)
-                            + B09 * K(8, c) + B10 * K(9, c) + B11 * K(1, c) + B12 * K(2, c);
+            const PtR k4 = PtR(B01) * K(0, c) + PtR(B06) * K(5, c) + PtR(B07) * K(6, c) + PtR(B08) * K(7, c)
+                         + PtR(B09) * K(8, c) + PtR(B10) * K(9, c) + PtR(B11) * K(1, c) + PtR(B12) * K(2, c);
             K(3, c) = k4;
-            dsf[c] = dt * k4;
-            sf[c] = si[c] + dsf[c];
-            sr[c] = P.atol + P.rtol * pt_max(fabs(si[c]), fabs(sf[c]));
+            const PtR d = dt * k4;
+            dsf[c] = d;
+            sf[c] = si[c] + d;
+            sr[c] = PtR(P.atol) + PtR(P.rtol) * pt_max(fabs(si[c]), fabs(sf[c]));
         }
 #ifndef PT_EXACT
         if (P.noise != 0.0) {            /* PT_CTL_NOISE: sr += 2 |dt| nu per group, */
@@ -397,7 +395,7 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
             for (int c = 0; c < 6; ++c) sr[c] += (c < 3) ? np_ : nm_;
         }
 #endif
-        double err3 = 0.0, err5 = 0.0;                          /* :426-437 */
+        PtR err3 = 0.0, err5 = 0.0;                             /* :426-437 */
 #ifndef PT_EXACT
 #pragma unroll
         for (int c = 0; c < 6; ++c) sr[c] = pt_rcp(sr[c]);     /* now 1/sr */
@@ -412,21 +410,22 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
 #endif
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            const double e = K(3, c) - BH1 * K(0, c) - BH2 * K(8, c) - BH3 * K(2, c);
-            const double q = PT_OVER_SR(e, c);
+            const PtR e = K(3, c) - PtR(BH1) * K(0, c) - PtR(BH2) * K(8, c) - PtR(BH3) * K(2, c);
+            const PtR q = PT_OVER_SR(e, c);
             err3 = err3 + q * q;
         }
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            const double e = ER01 * K(0, c) + ER06 * K(5, c) + ER07 * K(6, c) + ER08 * K(7, c)
-                           + ER09 * K(8, c) + ER10 * K(9, c) + ER11 * K(1, c) + ER12 * K(2, c);
-            const double q = PT_OVER_SR(e, c);
+            const PtR e = PtR(ER01) * K(0, c) + PtR(ER06) * K(5, c) + PtR(ER07) * K(6, c) + PtR(ER08) * K(7, c)
+                        + PtR(ER09) * K(8, c) + PtR(ER10) * K(9, c) + PtR(ER11) * K(1, c) + PtR(ER12) * K(2, c);
+            const PtR q = PT_OVER_SR(e, c);
             err5 = err5 + q * q;
         }
 #undef PT_OVER_SR
         const double deno = err5 + 1.0e-02 * err3;
 #ifdef PT_EXACT
-        return (deno <= 0.0) ? fabs(dt) * err5 / sqrt(6.0) : fabs(dt) * err5 / sqrt(6.0 * deno);
+        const double num = PtR(fabs(dt)) * err5;
+        return num / sqrt((deno <= 0.0) ? 6.0 : (double)(PtR(6.0) * deno));
 #else
         /* 1/sqrt(6) = 0.40824829046386307; the refined reciprocal square
          * root outside the subnormal range of its hardware approximation */
@@ -447,11 +446,11 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
 #ifdef PT_EXACT
-            double a = 0.0, e = 0.0;
-            a = a + CK_C1 * K(0, c); a = a + CK_C2 * K(1, c); a = a + CK_C3 * K(2, c);
-            a = a + CK_C4 * K(3, c); a = a + CK_C5 * K(4, c); a = a + CK_C6 * K(5, c);
-            e = e + CK_D1 * K(0, c); e = e + CK_D2 * K(1, c); e = e + CK_D3 * K(2, c);
-            e = e + CK_D4 * K(3, c); e = e + CK_D5 * K(4, c); e = e + CK_D6 * K(5, c);
+            PtR a = 0.0, e = 0.0;
+            a = a + PtR(CK_C1) * K(0, c); a = a + PtR(CK_C2) * K(1, c); a = a + PtR(CK_C3) * K(2, c);
+            a = a + PtR(CK_C4) * K(3, c); a = a + PtR(CK_C5) * K(4, c); a = a + PtR(CK_C6) * K(5, c);
+            e = e + PtR(CK_D1) * K(0, c); e = e + PtR(CK_D2) * K(1, c); e = e + PtR(CK_D3) * K(2, c);
+            e = e + PtR(CK_D4) * K(3, c); e = e + PtR(CK_D5) * K(4, c); e = e + PtR(CK_D6) * K(5, c);
 #else
             /* c2 = c5 = d2 = 0 (:94-97): the zero terms change nothing but
              * the sign of a zero sum, so the other builds leave them out
@@ -464,7 +463,7 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
             dsf[c] = a;
             sf[c] = si[c] + a;
 #ifdef PT_EXACT
-            const double sr = fabs(si[c]) + fabs(K(0, c)) + 2.2250738585072014e-308;
+            const double sr = PtR(fabs(si[c])) + fabs(K(0, c)) + 2.2250738585072014e-308;
 #else
             /* + DBL_MIN only changes a zero sum: test the bits instead (integer pipe) */
             double sr = fabs(si[c]) + fabs(K(0, c));
@@ -718,7 +717,7 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                     for (int c = 0; c < 6; ++c) K(dst, c) = a[c];
                 } else {
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) K(dst, c) = L.dt * a[c];    /* :137 */
+                    for (int c = 0; c < 6; ++c) K(dst, c) = PtR(L.dt) * a[c];    /* :137 */
                 }
             }
         } else {
@@ -849,7 +848,7 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                 } else {
                     if (METHOD == PT_METHOD_RK5) {
 #pragma unroll
-                        for (int c = 0; c < 6; ++c) K(0, c) = L.dt * K(T::F1, c);   /* :137, j = 1 */
+                        for (int c = 0; c < 6; ++c) K(0, c) = PtR(L.dt) * K(T::F1, c);   /* :137, j = 1 */
                     }
                 }
             }
