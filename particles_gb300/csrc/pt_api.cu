@@ -297,6 +297,8 @@ void attach_fields(const pt_fields *f, PtRun &R)
            : f->precision == PT_PREC_FP32 ? nbk * 512                 /* compact bricks */
            : f->nodes;
     R.oob = f->scratch + 2;
+    R.hand.ctl = f->scratch + 3;
+    R.hand.rec = reinterpret_cast<double *>(f->scratch + 32);
 }
 
 int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
@@ -327,7 +329,7 @@ int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
         e = cudaMemsetAsync(d_status, 0xff, (size_t)np * sizeof(int32_t), s);
         if (e != cudaSuccess) return cuda_err(e, "status reset");
     }
-    e = cudaMemsetAsync(f->scratch, 0, 3 * sizeof(unsigned long long), s);
+    e = cudaMemsetAsync(f->scratch, 0, 5 * sizeof(unsigned long long), s);
     if (e != cudaSuccess) return cuda_err(e, "scratch reset");
     e = launch_run(method, f, R, s);
     if (e != cudaSuccess) return cuda_err(e, "kernel launch");
@@ -389,7 +391,7 @@ extern "C" int pt_autotune(int32_t method, int64_t np, int32_t m, const pt_field
         R.block = kBlocks[bi];
         e = cudaMemcpy2DAsync(t_state, (size_t)mt * 64, d_state, (size_t)m * 64, 64, (size_t)ns,
                               cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(f->scratch, 0, 3 * sizeof(unsigned long long), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(f->scratch, 0, 5 * sizeof(unsigned long long), s);
         if (e == cudaSuccess) e = cudaEventRecord(ev[0], s);
         if (e == cudaSuccess) e = launch_run(method, f, R, s);
         if (e == cudaSuccess) e = cudaEventRecord(ev[1], s);

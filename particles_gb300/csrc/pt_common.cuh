@@ -21,6 +21,27 @@
 #include "pt_detmath.h"
 #include "pt_smul.h"
 
+/* Particles handed from the lane-per-particle machine to the eight-lane one
+ * (pt_coop.cuh) when a launch runs out of queued particles: ctl[0] counts the
+ * records, ctl[1] is the head they are taken from; a record holds a particle
+ * between two attempts. */
+#define PT_HAND_WORDS 22
+/* 16 warps on each of 152 SMs with PT_HAND_LANES particles each; a warp that
+ * finds the list full keeps its particles */
+#define PT_HAND_CAP 32768
+/* Lanes a warp still has at work when it hands over.  One lane per particle
+ * costs a scheduler ~2,500 FP64 slots per attempt for up to 32 particles,
+ * eight lanes ~900 for 4: equal at about 11.  Measured, exact build, 65,536
+ * particles, never / 4 / 8 / 12 / 16 / 24: DOP853 25.3 / 21.9 / 20.2 / 20.0 /
+ * 26.8 / 29.2 ms, RK5 21.4 / 18.3 / 17.3 / 17.2 / 23.9 / 26.0 ms. */
+#ifndef PT_HAND_LANES
+#define PT_HAND_LANES 12
+#endif
+struct PtHand {
+    unsigned long long *ctl;  /* 2 words, zeroed before a launch; NULL: no hand-over */
+    double *rec;              /* PT_HAND_WORDS words per record */
+};
+
 /* Everything a particle-integration kernel reads, by value in the launch. */
 struct PtRun {
     /* params(1:17) unpacked as integrations.F90:103-118,330-346 */
@@ -79,6 +100,7 @@ struct PtRun {
     int32_t *work;         /* per particle: attempts made in this run, or NULL */
     const int64_t *qlen;   /* ensembles: device queue length (else np) */
     const double *tstop;   /* ensembles: device window end (else tend) */
+    PtHand hand;
 };
 
 /* Launch variant of an integrator: the same kernel compiled with the

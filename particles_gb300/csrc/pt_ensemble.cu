@@ -39,6 +39,7 @@ struct pt_ensemble {
     PtRun *d_tab;
     double *d_tstop;
     int32_t *d_flags;
+    PtHand hand;                /* one allocation, ctl first */
     EnsBufs B;
     cudaGraph_t graph;
     cudaGraphExec_t exec;
@@ -72,8 +73,9 @@ __global__ void k_ens_init(EnsBufs B)
 }
 
 /* Before a window: queue heads to 0, the queue length to the compacted one. */
-__global__ void k_ens_reset(EnsBufs B)
+__global__ void k_ens_reset(EnsBufs B, unsigned long long *hand)
 {
+    if (threadIdx.x < 2) hand[threadIdx.x] = 0ull;
     const int k = threadIdx.x / PT_ENS_CTL, w = threadIdx.x % PT_ENS_CTL;
     if (k >= B.nmem) return;
     unsigned long long *c = B.ctl + (int64_t)k * PT_ENS_CTL;
@@ -213,7 +215,7 @@ static cudaError_t ens_launch(const pt_ensemble *e, int64_t ntot, cudaStream_t s
 static cudaError_t ens_window(pt_ensemble *e, cudaStream_t s)
 {
     const EnsBufs &B = e->B;
-    k_ens_reset<<<1, PT_ENS_CTL * PT_ENSEMBLE_MAX, 0, s>>>(B);
+    k_ens_reset<<<1, PT_ENS_CTL * PT_ENSEMBLE_MAX, 0, s>>>(B, e->hand.ctl);
     cudaError_t err = ens_launch(e, e->ntot, s);
     if (err != cudaSuccess) return err;
     const dim3 grid(ens_grid(e->npmax), e->nmem);
@@ -232,6 +234,7 @@ static void ens_free(pt_ensemble *e)
     cudaFree(e->d_tab);
     cudaFree(e->d_tstop);
     cudaFree(e->d_flags);
+    cudaFree(e->hand.ctl);
     cudaFree(e->B.ctl);
     cudaFree(e->B.idx);
     delete e;
@@ -281,6 +284,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
     }
     pt_ensemble *e = new pt_ensemble();
     memset(&e->B, 0, sizeof e->B);
+    e->hand.ctl = nullptr;
     e->method = method;
     e->precision = prec;
     e->nc = prec == PT_PREC_FP32 ? f0->nc32 : (prec == PT_PREC_BF16 ? f0->nc16 : f0->nc);
@@ -292,6 +296,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
     cudaError_t err = cudaMalloc(&e->d_tab, sizeof(PtRun) * nmembers);
     if (err == cudaSuccess) err = cudaMalloc(&e->d_tstop, sizeof(double));
     if (err == cudaSuccess) err = cudaMalloc(&e->d_flags, 16);   /* flags, out-of-range count */
+    if (err == cudaSuccess) err = cudaMalloc(&e->hand.ctl, 256 + (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8);
     if (err == cudaSuccess) err = cudaMalloc(&e->B.ctl, sizeof(unsigned long long) * PT_ENS_CTL * nmembers);
     if (err == cudaSuccess) err = cudaMalloc(&e->B.idx, sizeof(int32_t) * (idx_elems > 0 ? idx_elems : 1));
     if (err != cudaSuccess) {
@@ -306,6 +311,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
         const int32_t tpb = pt_opt_threads_per_block(opt);
         e->block = tpb ? tpb : ((t >> 8) ? (t >> 8) : PT_BLOCK_DEFAULT);
     }
+    e->hand.rec = reinterpret_cast<double *>(e->hand.ctl + 32);
     int64_t off = 0;
     for (int k = 0; k < nmembers; ++k) {
         const pt_member &M = members[k];
@@ -325,6 +331,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
         R.work = e->B.idx + off + 3 * M.np;
         R.tstop = e->d_tstop;
         R.flags = e->d_flags;
+        R.hand = e->hand;
         R.oob = reinterpret_cast<unsigned long long *>(e->d_flags + 2);
         R.minb = e->minb;
         R.block = e->block;

@@ -31,6 +31,9 @@
 #include "pt_common.cuh"
 #include "pt_detmath.h"
 #include "pt_integrator.cuh"
+#ifdef PT_EXACT
+#include "pt_coop.cuh"
+#endif
 
 #ifndef PT_SFX
 #error "PT_SFX must be defined (exact or fma)"
@@ -237,23 +240,144 @@ struct EvalF64 {
     }
 };
 
+#ifdef PT_EXACT
+/* f(s) with eight lanes per particle (pt_coop.cuh): the operations of
+ * EvalF64::f, each component's in the same order.  s is the lane's component
+ * of the stage state, the result its component of f.  tr: the group's
+ * transpose area. */
+template <int NC>
+struct CoopF64 : EvalF64<NC> {
+    static constexpr int NV = (NC == 10) ? 9 : 6;
+    static constexpr int kCoopRows = NV;
+    struct CoopOrigin {};
+    static __device__ __forceinline__ void coop_begin(const PtRun &, const pt_sm::Group &, double,
+                                                      CoopOrigin &) {}
+    static __device__ __forceinline__ double coop_f(const PtRun &P, const pt_sm::Group &G, double *tr,
+                                                    double s, double, const CoopOrigin &)
+    {
+        /* the cell and offset of the lane's axis (lanes 0-2; the others' values are unused) */
+        const PtR x = P.unit_map ? s : pt_qdiv(pt_fsub(s, P.xl[G.ax]), P.xs[G.ax], P.inv_xs[G.ax]);
+        const PtR xr = x + P.inv_dm[G.ax];
+        PtR xp = P.dmr[G.ax] * (xr - pt_floor(xr));
+        const int32_t r = pt_node_index(pt_floor(xp), P.dm[G.ax]);
+        xp = P.dmr[G.ax] * (x - pt_floor(x));
+        const PtR pl = pt_floor(xp);
+        const int32_t l = pt_node_index(pl, P.dm[G.ax]);
+        const double xd = xp - pl;
+        const double xu = PtR(1.0) - xd;
+        /* lane q's corner: x from bit 2, y from bit 1, z from bit 0 of q; an
+         * index fits 16 bits (dm <= 2^16) */
+        const uint32_t lr = (uint32_t)l | ((uint32_t)r << 16);
+        int32_t ix[3];
+        PtR w;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const bool right = (G.gl >> (2 - i)) & 1;
+            const uint32_t v = G.get(lr, i);
+            ix[i] = (int32_t)(right ? v >> 16 : v & 0xffffu);
+            const double d = G.get(xd, i), u = G.get(xu, i);
+            const double f = right ? d : u;
+            w = (i == 0) ? PtR(f) : w * f;
+        }
+        const int64_t d1 = P.dm[0], d12 = (int64_t)P.dm[0] * P.dm[1];
+        int64_t node = ix[0] + d1 * ix[1] + d12 * ix[2];
+        if (P.near) node = G.get(node, 0);
+        double v[NC];
+        load_rec<NC>(P.fld, PT_CHK(P, node, P.nrec), v);
+        /* gamma and the velocity of the lane's momentum while the records arrive */
+        const double ss = pt_fmul(s, s);
+        const double g = sqrt(PtR(G.get(ss, 3)) + G.get(ss, 4) + G.get(ss, 5) + 1.0);
+        const double vel = pt_qdiv(s, g, 1.0 / g);
+        const double vp = G.get(vel, G.gl + 3);               /* lanes 0-2: the axis' velocity */
+        double acc, acc8 = 0.0;
+        if (P.near) {
+            acc = v[0];
+#pragma unroll
+            for (int c = 1; c < (NV < 8 ? NV : 8); ++c) acc = (G.gl == c) ? v[c] : acc;
+            if (NV == 9) acc8 = v[8 % NC];
+        } else {
+            __syncwarp(G.mask);                                /* the last use of tr is over */
+#pragma unroll
+            for (int c = 0; c < NV; ++c) tr[c * 9 + G.gl] = w * v[c];
+            __syncwarp(G.mask);
+            const double *t = tr + (NV == 9 ? G.gl : G.c) * 9;
+            PtR a = t[0], b = 0.0;
+#pragma unroll
+            for (int k = 1; k < 8; ++k) a = a + t[k];
+            if (NV == 9) {
+                b = tr[8 * 9];
+#pragma unroll
+                for (int k = 1; k < 8; ++k) b = b + tr[8 * 9 + k];
+            }
+            acc = a;
+            acc8 = b;
+        }
+        const double U = G.get(acc, G.ax);
+        const double wv = pt_fsub(vel, U);                     /* lanes 3-5: v - U */
+        const int i1 = 3 + (G.ax == 2 ? 0 : G.ax + 1), i2 = 3 + (G.ax == 0 ? 2 : G.ax - 1);
+        const double w1 = G.get(wv, i1), w2 = G.get(wv, i2);
+        const double b1 = G.get(acc, i1), b2 = G.get(acc, i2);
+        /* lanes 0-2: v / vun by pt_qdiv's three operations; lanes 3-5: w1 b2 - w2 b1 */
+        const bool pos = G.gl < 3;
+        const double p1 = pt_fmul(pos ? vp : w1, pos ? P.inv_vun : b2);
+        const double p2 = __fma_rn(pos ? -P.vun : w2, pos ? p1 : b1, pos ? vp : -0.0);
+        double a = __fma_rn(pos ? p2 : -p2, pos ? P.inv_vun : 1.0, p1);
+        if (pos) {
+            const uint32_t e = (uint32_t)((unsigned long long)__double_as_longlong(p1) >> 52) & 0x7ffu;
+            const uint32_t ea = (uint32_t)((unsigned long long)__double_as_longlong(vp) >> 52) & 0x7ffu;
+            if (e - 63u > 1920u || ea < 116u) a = vp / P.vun;  /* pt_qdiv's excluded quotients */
+        }
+        double f = a;
+        if (NV == 9) {
+            const double j0 = G.get(acc, 6), j1 = G.get(acc, 7);
+            f = PtR(f) + PtR(P.eta) * (G.ax == 0 ? j0 : (G.ax == 1 ? j1 : acc8));
+        }
+        f = pt_fmul(P.qom, f);
+        return pos ? a : f;
+    }
+};
+
+template <int METHOD, int NC>
+__global__ void __launch_bounds__(128, 3) k_coop(const PtRun P, bool from_queue)
+{
+    pt_sm::run_coop<METHOD, CoopF64<NC>>(pt_sm::Members<false>{ P }, from_queue);
+}
+
+template <int METHOD, int NC>
+__global__ void __launch_bounds__(128, 3) k_ensemble_coop(const PtRun *__restrict__ tab, int nmem,
+                                                          int64_t few)
+{
+    __shared__ PtRun sP[PT_ENS_MAX];
+    __shared__ int64_t sN[PT_ENS_MAX];
+    pt_sm::ens_load(tab, nmem, sP, sN);
+    const pt_sm::Members<true> MB{ sP, sN, nmem };
+    pt_sm::run_coop<METHOD, CoopF64<NC>, true>(MB, MB.total() <= few);
+}
+constexpr bool kHand = true;
+#else
+constexpr bool kHand = false;
+#endif
+
+
 template <int METHOD, int NC, bool LEARN, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
 k_integrate(const PtRun P)
 {
-    pt_sm::run_machine<METHOD, EvalF64<NC>, LEARN>(pt_sm::Members<false>{ P });
+    pt_sm::run_machine<METHOD, EvalF64<NC>, LEARN, false, kHand && !LEARN>(pt_sm::Members<false>{ P });
 }
 
 /* Several runs (members: snapshots, tolerances, particle sets) in one
  * persistent launch; every lane drains the members' queues in table order. */
 template <int METHOD, int NC, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
-k_ensemble(const PtRun *__restrict__ tab, int nmem)
+k_ensemble(const PtRun *__restrict__ tab, int nmem, int64_t few)
 {
     __shared__ PtRun sP[PT_ENS_MAX];
     __shared__ int64_t sN[PT_ENS_MAX];
     pt_sm::ens_load(tab, nmem, sP, sN);
-    pt_sm::run_machine<METHOD, EvalF64<NC>, false, true>(pt_sm::Members<true>{ sP, sN, nmem });
+    const pt_sm::Members<true> MB{ sP, sN, nmem };
+    if (kHand && MB.total() <= few) return;        /* k_ensemble_coop takes the queue */
+    pt_sm::run_machine<METHOD, EvalF64<NC>, false, true, kHand>(MB);
 }
 
 /* Standalone f(vec) for parity tests of the gather and force. */
@@ -306,9 +430,14 @@ cudaError_t launch_ens1(const PtRun *tab, int nmem, int block, int64_t ntot, cud
 {
     static int cache[2] = { -1, 1 };
     const int smem = pt_sm::smem_bytes<METHOD>(block, false);
+#ifdef PT_EXACT
+    const int64_t few = (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+#else
+    const int64_t few = 0;
+#endif
     return pt_sm::launch_persistent(k_ensemble<METHOD, NC, MINB>, block, smem,
                                     pt_sm::smem_bytes<METHOD>(PT_BLOCK_MAX, false), cache, ntot, s,
-                                    tab, nmem);
+                                    tab, nmem, few);
 }
 
 template <int METHOD, int NC>
@@ -317,11 +446,20 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
 {
     if (ntot == 0) return cudaSuccess;          /* ntot < 0: configure only */
     if (!block) block = PT_BLOCK_DEFAULT;
+    cudaError_t e;
     switch (minb) {
-    case 2: return launch_ens1<METHOD, NC, 2>(tab, nmem, block, ntot, s);
-    case 4: return launch_ens1<METHOD, NC, 4>(tab, nmem, block, ntot, s);
-    default: return launch_ens1<METHOD, NC, 3>(tab, nmem, block, ntot, s);
+    case 2: e = launch_ens1<METHOD, NC, 2>(tab, nmem, block, ntot, s); break;
+    case 4: e = launch_ens1<METHOD, NC, 4>(tab, nmem, block, ntot, s); break;
+    default: e = launch_ens1<METHOD, NC, 3>(tab, nmem, block, ntot, s); break;
     }
+#ifdef PT_EXACT
+    /* how many particles are left is known on the device only: both kernels
+     * are launched, and the one that is not to take the queue finds nothing */
+    if (e == cudaSuccess && ntot > 0)
+        e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_ensemble_coop<METHOD, NC>, -1, s, tab, nmem,
+                                                    (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
+#endif
+    return e;
 }
 
 template <int METHOD, int NC, bool LEARN>
@@ -338,6 +476,15 @@ template <int METHOD, int NC>
 cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
+#ifdef PT_EXACT
+    if (!P.mlp && !P.rec) {
+        const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+        cudaError_t e = few ? cudaSuccess : launch_v<METHOD, NC, false>(P, s);
+        if (e == cudaSuccess && (few || P.hand.ctl))
+            e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC>, few ? P.np : -1, s, P, few);
+        return e;
+    }
+#endif
     return (P.mlp || P.rec) ? launch_v<METHOD, NC, true>(P, s) : launch_v<METHOD, NC, false>(P, s);
 }
 

@@ -192,6 +192,30 @@ __device__ __forceinline__ void lane_close(const PtRun &P, const KRows &K, const
     if (st == PT_ST_TIMEOUT) atomicExch(P.flags, 1);
 }
 
+/* A handed-over particle (PtHand): word by word what the next attempt needs. */
+struct HandRec {
+    enum { T, DT, ERROLD, SI, K1 = SI + 6, C0 = K1 + 6, C1, C2, P, START, N_W0, FLAGS, WORDS };
+};
+static_assert(HandRec::WORDS == PT_HAND_WORDS, "hand-over record size");
+
+template <int METHOD>
+__device__ __forceinline__ void lane_hand(double *r, const KRows &K, const Lane &L,
+                                          const double si[6], uint64_t t_start, int mi)
+{
+    long long *w = reinterpret_cast<long long *>(r);
+    r[HandRec::T] = L.t; r[HandRec::DT] = L.dt; r[HandRec::ERROLD] = L.errold;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        r[HandRec::SI + c] = si[c];
+        r[HandRec::K1 + c] = K(Traits<METHOD>::F1, c);
+    }
+    w[HandRec::C0] = L.c0; w[HandRec::C1] = L.c1; w[HandRec::C2] = L.c2;
+    w[HandRec::P] = L.p;
+    w[HandRec::START] = (long long)t_start;
+    w[HandRec::N_W0] = ((long long)L.w0 << 32) | (uint32_t)L.n;
+    w[HandRec::FLAGS] = (L.rejected ? 1 : 0) | (mi << 1);
+}
+
 /* Status before an attempt: PT_GO = go on, else the particle closes. */
 __device__ __forceinline__ int32_t lane_check(const PtRun &P, const Lane &L, uint64_t t_start)
 {
@@ -614,12 +638,20 @@ template <> struct Members<true> {
     const PtRun *tab;        /* shared memory */
     const int64_t *nq;       /* shared memory: queue length per member */
     int n;
+    __device__ __forceinline__ int64_t total() const
+    {
+        int64_t t = 0;
+        for (int k = 0; k < n; ++k) t += nq[k];
+        return t;
+    }
     __device__ __forceinline__ const PtRun &q(int mi) const { return tab[mi]; }
     __device__ __forceinline__ int64_t queue_len(int mi) const { return nq[mi]; }
     __device__ __forceinline__ int count() const { return n; }
 };
 
-template <int METHOD, class EV, bool LEARN, bool ENS = false>
+/* HAND: when the queue has run dry and at most kHandLanes lanes of a warp
+ * still integrate, their particles go to the hand-over list. */
+template <int METHOD, class EV, bool LEARN, bool ENS = false, bool HAND = false>
 __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
 {
     using T = Traits<METHOD>;
@@ -852,9 +884,25 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                     }
                 }
             }
-            if (!__any_sync(0xffffffffu, active)) {
+            const unsigned act = __ballot_sync(0xffffffffu, active);
+            if (!act) {
                 if (!__any_sync(0xffffffffu, !drained)) break;
                 continue;                                               /* j stays 0 */
+            }
+            if (HAND && __popc(act) <= PT_HAND_LANES && __any_sync(0xffffffffu, drained)) {
+                const PtHand H = MB.q(0).hand;
+                if (H.ctl) {
+                    const int lane = threadIdx.x & 31;
+                    unsigned long long at = 0;
+                    if (lane == 0) at = atomicAdd(H.ctl, (unsigned long long)__popc(act));
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if (at + __popc(act) <= PT_HAND_CAP) {
+                        at += __popc(act & ((1u << lane) - 1u));
+                        if (active) lane_hand<METHOD>(H.rec + at * PT_HAND_WORDS, K, L, si, t_start, mi);
+                        break;
+                    }
+                    if (lane == 0) atomicAdd(H.ctl, 0ULL - (unsigned long long)__popc(act));
+                }
             }
         }
         j = (j + 1 < T::SLOTS) ? j + 1 : 0;

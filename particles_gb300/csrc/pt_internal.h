@@ -44,7 +44,8 @@ struct pt_fields {
     int32_t nb[3];              /* bricks per axis */
     int32_t nc16;               /* BF16 record width: 8 or 16 */
     int64_t bytes;
-    unsigned long long *scratch;   /* [0] queue head, [1] flags (2 x int32) */
+    unsigned long long *scratch;   /* [0] queue head, [1] flags (2 x int32), [2] out-of-range
+                                      count, [3..4] PtHand.ctl, [32..] PtHand.rec */
     unsigned char *ws;          /* host-buffer runs: device copies, reused across calls */
     size_t ws_bytes;
     unsigned char *pack;        /* host-buffer runs: the output rows a call wrote, packed */
