@@ -18,7 +18,9 @@
  *   - the force runs on lanes 3-5 while lanes 0-2 divide by vun.
  * Every component sees the same operations on the same operands in the same
  * order as in pt_integrator.cuh, so a particle's bits do not depend on which
- * machine integrated it.
+ * machine integrated it.  In the non-exact builds that includes which product
+ * of a sum the compiler contracts there; where its choice is not the only one
+ * it is written out here (tests/test_gpu_coop.py compares the two machines).
  */
 #ifndef PT_COOP_CUH
 #define PT_COOP_CUH
@@ -169,10 +171,32 @@ __device__ __forceinline__ void coop_row(const Group &G, double t, double dt, do
     const double ds = sf - si;
     const double a = scale ? dt * ka : ka;
     const double b = scale ? dt * kb : kb;
+#ifdef PT_EXACT
     const double st = fr * si + fl * sf + fl * fr * ((a - ds) * fr + (ds - b) * fl);
+#else
+    /* which of two products contracts as in dense_row */
+    const double in = scale ? fma(a - ds, fr, __dmul_rn(ds - b, fl)) : (a - ds) * fr + (ds - b) * fl;
+    const double st = fr * si + fl * sf + fl * fr * in;
+#endif
     const double s3 = G.get(st, 3), s4 = G.get(st, 4), s5 = G.get(st, 5);
     const double gam = sqrt(s3 * s3 + s4 * s4 + s5 * s5 + 1.0);
     row[G.gl] = G.gl < 6 ? st : (G.gl == 6 ? gam : dt);
+}
+
+/* s = si + d with the increment d = h k.  The non-exact builds' lane-per-
+ * particle machine contracts the two where the increment itself is not used
+ * (the FMA build), and rounds it where it is (DELTA); so do these lanes. */
+template <bool DELTA>
+__device__ __forceinline__ void coop_step(double h, double k, double si, double &s, double &d)
+{
+#ifdef PT_EXACT
+    const PtR x = PtR(h) * k;
+    d = x;
+    s = si + x;
+#else
+    d = __dmul_rn(h, k);
+    s = DELTA ? __dadd_rn(si, d) : fma(h, k, si);
+#endif
 }
 
 /* The lane's component of the stage state and its increment, as stage_state. */
@@ -183,16 +207,11 @@ __device__ __forceinline__ void coop_stage(int j, const KOwn &K, double si, doub
     if (METHOD == PT_METHOD_DOP853) {
         const Stage &S = kDop[j];
         if (j == 1) {
-            const PtR h = PtR(dt) * S.a[0];
-            const PtR d = h * K(0);
-            dl = d;
-            ss = si + d;
+            coop_step<DELTA>(PtR(dt) * S.a[0], K(0), si, ss, dl);
         } else {
             PtR acc = PtR(S.a[0]) * K(S.r[0]);
             for (int i = 1; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i]);
-            const PtR d = dt * acc;
-            dl = d;
-            ss = si + d;
+            coop_step<DELTA>(dt, acc, si, ss, dl);
         }
     } else {
         const Stage &S = kCk[j];
@@ -209,56 +228,91 @@ __device__ __forceinline__ void coop_stage(int j, const KOwn &K, double si, doub
     }
 }
 
+#ifndef PT_EXACT
+/* The largest |v| of the lane's group of components (positions, momenta). */
+__device__ __forceinline__ double coop_group_max(const Group &G, double v)
+{
+    const int b = G.c < 3 ? 0 : 3;
+    const double a = fabs(v);
+    const double v0 = G.get(a, b), v1 = G.get(a, b + 1), v2 = G.get(a, b + 2);
+    return pt_max(v0, pt_max(v1, v2));
+}
+#endif
+
 /* Final combination and error norm, as finish_attempt: sf, dsf of the lane's
  * component; the norm on every lane. */
-template <int METHOD>
+template <int METHOD, bool DELTA>
 __device__ __forceinline__ double coop_finish(const PtRun &P, const Group &G, const KOwn &K,
                                               double si, double dt, double &sf, double &dsf)
 {
     if (METHOD == PT_METHOD_DOP853) {
         const PtR k4 = PtR(B01) * K(0) + PtR(B06) * K(5) + PtR(B07) * K(6) + PtR(B08) * K(7)
                      + PtR(B09) * K(8) + PtR(B10) * K(9) + PtR(B11) * K(1) + PtR(B12) * K(2);
-        const PtR d = dt * k4;
-        dsf = d;
-        sf = si + d;
-        const double sr = PtR(P.atol) + PtR(P.rtol) * pt_max(fabs(si), fabs(sf));
+        coop_step<DELTA>(dt, k4, si, sf, dsf);
+        double sr = PtR(P.atol) + PtR(P.rtol) * pt_max(fabs(si), fabs(sf));
         const PtR e3 = k4 - PtR(BH1) * K(0) - PtR(BH2) * K(8) - PtR(BH3) * K(2);
         const PtR e5 = PtR(ER01) * K(0) + PtR(ER06) * K(5) + PtR(ER07) * K(6) + PtR(ER08) * K(7)
                      + PtR(ER09) * K(8) + PtR(ER10) * K(9) + PtR(ER11) * K(1) + PtR(ER12) * K(2);
+#ifdef PT_EXACT
         const double ysr = 1.0 / sr;
         const PtR q3 = pt_qdiv(e3, sr, ysr), q5 = pt_qdiv(e5, sr, ysr);
-        const double s3 = q3 * q3, s5 = q5 * q5;
+        const double t3 = q3 * q3, t5 = q5 * q5;       /* squared before they are handed round */
+#else
+        if (P.noise != 0.0) sr = fma(P.noise, coop_group_max(G, dsf), sr);
+        const double ysr = pt_rcp(sr);
+        const double t3 = e3 * ysr, t5 = e5 * ysr;
+#endif
         /* the two sums side by side: err3 on even lanes, err5 on odd ones */
-        PtR s;
+        PtR s = 0.0;
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
-            const double a = G.get(s3, i), b = G.get(s5, i);
+            const double a = G.get(t3, i), b = G.get(t5, i);
             const double v = (G.gl & 1) ? b : a;
+#ifdef PT_EXACT
             s = (i == 0) ? PtR(v) : s + v;
+#else
+            s = (i == 0) ? v : (i == 1) ? fma(s, s, __dmul_rn(v, v)) : fma(v, v, s);
+#endif
         }
         const PtR err3 = G.get((double)s, 0), err5 = G.get((double)s, 1);
         const double deno = err5 + 1.0e-02 * err3;
+#ifdef PT_EXACT
         const double num = PtR(fabs(dt)) * err5;
         return num / sqrt((deno <= 0.0) ? 6.0 : (double)(PtR(6.0) * deno));
+#else
+        if (!(deno > 1.0e-300))
+            return (deno <= 0.0) ? fabs(dt) * err5 * 0.40824829046386307
+                                 : fabs(dt) * err5 / sqrt(6.0 * deno);
+        return fabs(dt) * err5 * pt_rsqrt(6.0 * deno);
+#endif
     } else {
+#ifdef PT_EXACT
         PtR a = 0.0, e = 0.0;
         a = a + PtR(CK_C1) * K(0); a = a + PtR(CK_C2) * K(1); a = a + PtR(CK_C3) * K(2);
         a = a + PtR(CK_C4) * K(3); a = a + PtR(CK_C5) * K(4); a = a + PtR(CK_C6) * K(5);
         e = e + PtR(CK_D1) * K(0); e = e + PtR(CK_D2) * K(1); e = e + PtR(CK_D3) * K(2);
         e = e + PtR(CK_D4) * K(3); e = e + PtR(CK_D5) * K(4); e = e + PtR(CK_D6) * K(5);
+        const double sr = PtR(fabs(si)) + fabs(K(0)) + 2.2250738585072014e-308;
+#else
+        const double a = CK_C1 * K(0) + CK_C3 * K(2) + CK_C4 * K(3) + CK_C6 * K(5);
+        const double e = CK_D1 * K(0) + CK_D3 * K(2) + CK_D4 * K(3) + CK_D5 * K(4) + CK_D6 * K(5);
+        double sr = fabs(si) + fabs(K(0));
+        if (P.noise != 0.0) sr += __dmul_rn(P.noise, coop_group_max(G, K(0)));
+        if (__double_as_longlong(sr) == 0) sr = 2.2250738585072014e-308;
+#endif
         dsf = a;
         sf = si + a;
-        const double sr = PtR(fabs(si)) + fabs(K(0)) + 2.2250738585072014e-308;
         /* the largest |e / sr| by its bits (NaN above infinity: it propagates) */
+        const double r = PT_DIV((double)e, sr);
         const unsigned long long q =
-            (unsigned long long)__double_as_longlong((double)e / sr) & 0x7fffffffffffffffULL;
+            (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffULL;
         unsigned long long del = G.get(q, 0);
 #pragma unroll
         for (int i = 1; i < 6; ++i) {
             const unsigned long long v = G.get(q, i);
             del = v > del ? v : del;
         }
-        return __longlong_as_double((long long)del) / P.atol;
+        return PT_DIV(__longlong_as_double((long long)del), P.atol);
     }
 }
 
@@ -286,12 +340,12 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
     int j = 0;
     for (;;) {
         double pt = si, dl = 0.0;
-        bool need = false, fresh = false;
+        bool need = false, fresh = false, handed_over = false;
         int mode = M_IDLE;
         double q = 0.0;
         if (j == 0) {
             if (active) {
-                q = coop_finish<METHOD>(PT_Q, G, K, si, L.dt, pt, dl);
+                q = coop_finish<METHOD, EV::kDelta>(PT_Q, G, K, si, L.dt, pt, dl);
                 if (q != q) {
                     coop_close<METHOD>(PT_Q, G, K, L, si, PT_ST_NONFINITE);
                     active = false;
@@ -327,6 +381,7 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
                     if (handed && qi < handed) {
                         coop_take<METHOD>(H.rec + qi * PT_HAND_WORDS, G, K, L, si, t_start, mi);
                         mode = M_READY;
+                        handed_over = true;
                         active = true;
                     } else {
                         drained = true;
@@ -418,6 +473,10 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
                 next_time(PT_Q, L);
             }
             if (active && (mode == M_ACCEPT || mode == M_READY)) EV::coop_begin(PT_Q, G, si, O);
+#ifndef PT_EXACT
+            /* a handed-over step is capped already */
+            if (PT_Q.face && active && !handed_over) L.dt = EV::coop_face_cap(PT_Q, G, si, O, L.dt);
+#endif
             if (active) {
                 int32_t st = lane_check(PT_Q, L, t_start);
                 st = G.get(st, 0);                  /* one clock reading for the group */

@@ -31,9 +31,7 @@
 #include "pt_common.cuh"
 #include "pt_detmath.h"
 #include "pt_integrator.cuh"
-#ifdef PT_EXACT
 #include "pt_coop.cuh"
-#endif
 
 #ifndef PT_SFX
 #error "PT_SFX must be defined (exact or fma)"
@@ -240,7 +238,6 @@ struct EvalF64 {
     }
 };
 
-#ifdef PT_EXACT
 /* f(s) with eight lanes per particle (pt_coop.cuh): the operations of
  * EvalF64::f, each component's in the same order.  s is the lane's component
  * of the stage state, the result its component of f.  tr: the group's
@@ -248,14 +245,27 @@ struct EvalF64 {
 template <int NC>
 struct CoopF64 : EvalF64<NC> {
     static constexpr int NV = (NC == 10) ? 9 : 6;
-    static constexpr int kCoopRows = NV;
     struct CoopOrigin {};
+#ifdef PT_EXACT
+    static constexpr int kCoopRows = NV;           /* products */
+#else
+    static constexpr int kCoopRows = NV + 1;       /* corner values, weights */
+    static __device__ __forceinline__ double coop_face_cap(const PtRun &P, const pt_sm::Group &G,
+                                                           double si, const CoopOrigin &, double h)
+    {
+        const float o = pt_sm::pt_cell_offset(P, si, G.ax), u = pt_d2f(si);
+        const float off[3] = { G.get(o, 0), G.get(o, 1), G.get(o, 2) };
+        const float um[3] = { G.get(u, 3), G.get(u, 4), G.get(u, 5) };
+        return pt_sm::pt_face_cap(P, off, um, h);
+    }
+#endif
     static __device__ __forceinline__ void coop_begin(const PtRun &, const pt_sm::Group &, double,
                                                       CoopOrigin &) {}
     static __device__ __forceinline__ double coop_f(const PtRun &P, const pt_sm::Group &G, double *tr,
                                                     double s, double, const CoopOrigin &)
     {
         /* the cell and offset of the lane's axis (lanes 0-2; the others' values are unused) */
+#ifdef PT_EXACT
         const PtR x = P.unit_map ? s : pt_qdiv(pt_fsub(s, P.xl[G.ax]), P.xs[G.ax], P.inv_xs[G.ax]);
         const PtR xr = x + P.inv_dm[G.ax];
         PtR xp = P.dmr[G.ax] * (xr - pt_floor(xr));
@@ -265,6 +275,20 @@ struct CoopF64 : EvalF64<NC> {
         const int32_t l = pt_node_index(pl, P.dm[G.ax]);
         const double xd = xp - pl;
         const double xu = PtR(1.0) - xd;
+#else
+        const double xn = fma(s, P.gsx[G.ax], P.gox[G.ax]);
+        const double fl = pt_floor(xn);
+        const int32_t ci = pt_i32(fl), dm = P.dm[G.ax], dmm = P.dm_mask[G.ax];
+        int32_t l;
+        if (dmm) {
+            l = ci & dmm;
+        } else {
+            l = ci % dm;
+            if (l < 0) l += dm;
+        }
+        const int32_t r = (l + 1 == dm) ? 0 : l + 1;
+        const double xd = xn - fl, xu = 1.0 - xd;
+#endif
         /* lane q's corner: x from bit 2, y from bit 1, z from bit 0 of q; an
          * index fits 16 bits (dm <= 2^16) */
         const uint32_t lr = (uint32_t)l | ((uint32_t)r << 16);
@@ -285,9 +309,15 @@ struct CoopF64 : EvalF64<NC> {
         double v[NC];
         load_rec<NC>(P.fld, PT_CHK(P, node, P.nrec), v);
         /* gamma and the velocity of the lane's momentum while the records arrive */
+#ifdef PT_EXACT
         const double ss = pt_fmul(s, s);
         const double g = sqrt(PtR(G.get(ss, 3)) + G.get(ss, 4) + G.get(ss, 5) + 1.0);
         const double vel = pt_qdiv(s, g, 1.0 / g);
+#else
+        const double s3 = G.get(s, 3), s4 = G.get(s, 4), s5 = G.get(s, 5);
+        const double ig = pt_sm::pt_rsqrt(fma(s3, s3, fma(s4, s4, fma(s5, s5, 1.0))));
+        const double vel = s * ig;
+#endif
         const double vp = G.get(vel, G.gl + 3);               /* lanes 0-2: the axis' velocity */
         double acc, acc8 = 0.0;
         if (P.near) {
@@ -297,10 +327,26 @@ struct CoopF64 : EvalF64<NC> {
             if (NV == 9) acc8 = v[8 % NC];
         } else {
             __syncwarp(G.mask);                                /* the last use of tr is over */
+#ifdef PT_EXACT
 #pragma unroll
             for (int c = 0; c < NV; ++c) tr[c * 9 + G.gl] = w * v[c];
+#else
+#pragma unroll
+            for (int c = 0; c < NV; ++c) tr[c * 9 + G.gl] = v[c];
+            tr[NV * 9 + G.gl] = w;
+#endif
             __syncwarp(G.mask);
             const double *t = tr + (NV == 9 ? G.gl : G.c) * 9;
+#ifndef PT_EXACT
+            const double *wt = tr + NV * 9;
+            double a = fma(wt[0], t[0], __dmul_rn(wt[1], t[1])), b = 0.0;
+            if (NV == 9) b = fma(wt[0], tr[8 * 9], __dmul_rn(wt[1], tr[8 * 9 + 1]));
+#pragma unroll
+            for (int k = 2; k < 8; ++k) {
+                a = fma(wt[k], t[k], a);
+                if (NV == 9) b = fma(wt[k], tr[8 * 9 + k], b);
+            }
+#else
             PtR a = t[0], b = 0.0;
 #pragma unroll
             for (int k = 1; k < 8; ++k) a = a + t[k];
@@ -309,16 +355,22 @@ struct CoopF64 : EvalF64<NC> {
 #pragma unroll
                 for (int k = 1; k < 8; ++k) b = b + tr[8 * 9 + k];
             }
+#endif
             acc = a;
             acc8 = b;
         }
         const double U = G.get(acc, G.ax);
+#ifdef PT_EXACT
         const double wv = pt_fsub(vel, U);                     /* lanes 3-5: v - U */
+#else
+        const double wv = vel - U;
+#endif
         const int i1 = 3 + (G.ax == 2 ? 0 : G.ax + 1), i2 = 3 + (G.ax == 0 ? 2 : G.ax - 1);
         const double w1 = G.get(wv, i1), w2 = G.get(wv, i2);
         const double b1 = G.get(acc, i1), b2 = G.get(acc, i2);
-        /* lanes 0-2: v / vun by pt_qdiv's three operations; lanes 3-5: w1 b2 - w2 b1 */
         const bool pos = G.gl < 3;
+#ifdef PT_EXACT
+        /* lanes 0-2: v / vun by pt_qdiv's three operations; lanes 3-5: w1 b2 - w2 b1 */
         const double p1 = pt_fmul(pos ? vp : w1, pos ? P.inv_vun : b2);
         const double p2 = __fma_rn(pos ? -P.vun : w2, pos ? p1 : b1, pos ? vp : -0.0);
         double a = __fma_rn(pos ? p2 : -p2, pos ? P.inv_vun : 1.0, p1);
@@ -333,6 +385,15 @@ struct CoopF64 : EvalF64<NC> {
             f = PtR(f) + PtR(P.eta) * (G.ax == 0 ? j0 : (G.ax == 1 ? j1 : acc8));
         }
         f = pt_fmul(P.qom, f);
+#else
+        const double a = vp * P.inv_vun;
+        double f = w1 * b2 - w2 * b1;
+        if (NV == 9) {
+            const double j0 = G.get(acc, 6), j1 = G.get(acc, 7);
+            f = fma(P.eta, G.ax == 0 ? j0 : (G.ax == 1 ? j1 : acc8), f);
+        }
+        f = P.qom * f;
+#endif
         return pos ? a : f;
     }
 };
@@ -353,17 +414,12 @@ __global__ void __launch_bounds__(128, 3) k_ensemble_coop(const PtRun *__restric
     const pt_sm::Members<true> MB{ sP, sN, nmem };
     pt_sm::run_coop<METHOD, CoopF64<NC>, true>(MB, MB.total() <= few);
 }
-constexpr bool kHand = true;
-#else
-constexpr bool kHand = false;
-#endif
-
 
 template <int METHOD, int NC, bool LEARN, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
 k_integrate(const PtRun P)
 {
-    pt_sm::run_machine<METHOD, EvalF64<NC>, LEARN, false, kHand && !LEARN>(pt_sm::Members<false>{ P });
+    pt_sm::run_machine<METHOD, EvalF64<NC>, LEARN, false, !LEARN>(pt_sm::Members<false>{ P });
 }
 
 /* Several runs (members: snapshots, tolerances, particle sets) in one
@@ -376,8 +432,8 @@ k_ensemble(const PtRun *__restrict__ tab, int nmem, int64_t few)
     __shared__ int64_t sN[PT_ENS_MAX];
     pt_sm::ens_load(tab, nmem, sP, sN);
     const pt_sm::Members<true> MB{ sP, sN, nmem };
-    if (kHand && MB.total() <= few) return;        /* k_ensemble_coop takes the queue */
-    pt_sm::run_machine<METHOD, EvalF64<NC>, false, true, kHand>(MB);
+    if (MB.total() <= few) return;        /* k_ensemble_coop takes the queue */
+    pt_sm::run_machine<METHOD, EvalF64<NC>, false, true, true>(MB);
 }
 
 /* Standalone f(vec) for parity tests of the gather and force. */
@@ -430,11 +486,7 @@ cudaError_t launch_ens1(const PtRun *tab, int nmem, int block, int64_t ntot, cud
 {
     static int cache[2] = { -1, 1 };
     const int smem = pt_sm::smem_bytes<METHOD>(block, false);
-#ifdef PT_EXACT
     const int64_t few = (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
-#else
-    const int64_t few = 0;
-#endif
     return pt_sm::launch_persistent(k_ensemble<METHOD, NC, MINB>, block, smem,
                                     pt_sm::smem_bytes<METHOD>(PT_BLOCK_MAX, false), cache, ntot, s,
                                     tab, nmem, few);
@@ -452,13 +504,11 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
     case 4: e = launch_ens1<METHOD, NC, 4>(tab, nmem, block, ntot, s); break;
     default: e = launch_ens1<METHOD, NC, 3>(tab, nmem, block, ntot, s); break;
     }
-#ifdef PT_EXACT
     /* how many particles are left is known on the device only: both kernels
      * are launched, and the one that is not to take the queue finds nothing */
     if (e == cudaSuccess && ntot > 0)
         e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_ensemble_coop<METHOD, NC>, -1, s, tab, nmem,
                                                     (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
-#endif
     return e;
 }
 
@@ -476,16 +526,12 @@ template <int METHOD, int NC>
 cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
-#ifdef PT_EXACT
-    if (!P.mlp && !P.rec) {
-        const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
-        cudaError_t e = few ? cudaSuccess : launch_v<METHOD, NC, false>(P, s);
-        if (e == cudaSuccess && (few || P.hand.ctl))
-            e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC>, few ? P.np : -1, s, P, few);
-        return e;
-    }
-#endif
-    return (P.mlp || P.rec) ? launch_v<METHOD, NC, true>(P, s) : launch_v<METHOD, NC, false>(P, s);
+    if (P.mlp || P.rec) return launch_v<METHOD, NC, true>(P, s);
+    const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+    cudaError_t e = few ? cudaSuccess : launch_v<METHOD, NC, false>(P, s);
+    if (e == cudaSuccess && (few || P.hand.ctl))
+        e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC>, few ? P.np : -1, s, P, few);
+    return e;
 }
 
 }  // namespace

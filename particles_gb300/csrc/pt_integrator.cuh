@@ -511,21 +511,18 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
  * -- plus the time to cross face_over of a cell along the fastest axis, so
  * the step ends just past that face.  FP32 suffices (an estimate; the error
  * norm still accepts or rejects the step). */
-__device__ __forceinline__ double pt_face_cap(const PtRun &P, const double si[6], double h)
+__device__ __forceinline__ double pt_face_cap(const PtRun &P, const float off[3], const float u[3],
+                                              double h)
 {
-    const float ux = pt_d2f(si[3]), uy = pt_d2f(si[4]), uz = pt_d2f(si[5]);
-    const float ig = rsqrtf(fmaf(ux, ux, fmaf(uy, uy, fmaf(uz, uz, 1.0f))));
-    const float u[3] = { ux, uy, uz };
+    const float ig = rsqrtf(fmaf(u[0], u[0], fmaf(u[1], u[1], fmaf(u[2], u[2], 1.0f))));
     const float th = P.face_skip * pt_d2f(h);
     float tmin = 3.0e38f, wmax = 0.0f;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const double xn = fma(si[i], P.gsx[i], P.gox[i]);
-        const float off = pt_d2f(xn - pt_floor(xn));               /* in [0, 1] */
         const float w = u[i] * ig * P.ivunf * P.gsxf[i];           /* cells per unit time */
         const float aw = fabsf(w);
         if (aw > 0.0f) {
-            const float d = (w > 0.0f) ? 1.0f - off : off;          /* cells to the next face */
+            const float d = (w > 0.0f) ? 1.0f - off[i] : off[i];    /* cells to the next face */
             /* first face on this axis at or after time th: d + k cells */
             const float k = fmaxf(0.0f, ceilf(fmaf(th, aw, -d)));
             tmin = fminf(tmin, (d + k) / aw);
@@ -534,6 +531,24 @@ __device__ __forceinline__ double pt_face_cap(const PtRun &P, const double si[6]
     }
     if (!(wmax > 0.0f)) return h;
     return pt_min(h, pt_f2d(tmin + P.face_over / wmax));
+}
+
+/* The offset in [0, 1] of x in its cell along axis i, in FP32. */
+__device__ __forceinline__ float pt_cell_offset(const PtRun &P, double x, int i)
+{
+    const double xn = fma(x, P.gsx[i], P.gox[i]);
+    return pt_d2f(xn - pt_floor(xn));
+}
+
+__device__ __forceinline__ double pt_face_cap(const PtRun &P, const double si[6], double h)
+{
+    float off[3], u[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        off[i] = pt_cell_offset(P, si[i], i);
+        u[i] = pt_d2f(si[3 + i]);
+    }
+    return pt_face_cap(P, off, u, h);
 }
 #endif
 

@@ -36,7 +36,7 @@
 
 #include "pt_common.cuh"
 #include "pt_convert.cuh"
-#include "pt_integrator.cuh"
+#include "pt_coop.cuh"
 
 #ifndef PT_PART
 #define PT_PART 0
@@ -274,19 +274,18 @@ struct EvalMixed {
         }
     }
 
-    /* f(s) with s = si + d: the stage position relative to the origin cell is
-     * off + d * dm / xs in FP32 (d is at most a few cells), the momentum
-     * u(si) + d in FP32; gather and force in FP32; every FP64 <-> FP32
-     * conversion on the integer pipe. */
-    static __device__ __forceinline__ void f(const PtRun &P, const double s[6], const double d[6],
-                                             const Origin &O, double a[6])
+    /* f(s) with s = si + d in FP32, d already rounded to it: the stage position
+     * relative to the origin cell is off + d * dm / xs (d is at most a few
+     * cells), the momentum u(si) + d; gather and force. */
+    static __device__ __forceinline__ void f32(const PtRun &P, const float d[6], const Origin &O,
+                                               float a[6])
     {
         constexpr int NV = G::NV;
         int32_t l[3], r[3];
         float xd[3], xu[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const float rel = fmaf(pt_d2f(d[i]), P.gsxf[i], O.off[i]);
+            const float rel = fmaf(d[i], P.gsxf[i], O.off[i]);
             const float cf = floorf(rel);
             xd[i] = rel - cf;
             const int32_t ci = O.cell[i] + (int32_t)cf;
@@ -307,17 +306,14 @@ struct EvalMixed {
                               pdu * xu[2], pdu * xd[2], pdd * xu[2], pdd * xd[2] };
         float acc[NV];
         G::gather(P, l, r, w8, acc);
-        /* the stage momentum in FP32: u(si) + the FP64 increment, both
-         * rounded to FP32 (the FP64 stage state s is not needed) */
-        const float ux = O.u[0] + pt_d2f(d[3]), uy = O.u[1] + pt_d2f(d[4]), uz = O.u[2] + pt_d2f(d[5]);
-        (void)s;
+        const float ux = O.u[0] + d[3], uy = O.u[1] + d[4], uz = O.u[2] + d[5];
         const float g = sqrtf(fmaf(ux, ux, fmaf(uy, uy, fmaf(uz, uz, 1.0f))));
         const float ig = 1.0f / g;
         const float v0 = ux * ig, v1 = uy * ig, v2 = uz * ig;
         const float w0 = v0 - acc[0], w1 = v1 - acc[1], w2 = v2 - acc[2];
-        a[0] = pt_f2d(v0 * P.ivunf);
-        a[1] = pt_f2d(v1 * P.ivunf);
-        a[2] = pt_f2d(v2 * P.ivunf);
+        a[0] = v0 * P.ivunf;
+        a[1] = v1 * P.ivunf;
+        a[2] = v2 * P.ivunf;
         float f3 = w1 * acc[5] - w2 * acc[4];
         float f4 = w2 * acc[3] - w0 * acc[5];
         float f5 = w0 * acc[4] - w1 * acc[3];
@@ -326,9 +322,60 @@ struct EvalMixed {
             f4 = fmaf(P.etaf, acc[7 % NV], f4);
             f5 = fmaf(P.etaf, acc[8 % NV], f5);
         }
-        a[3] = pt_f2d(P.qomf * f3);
-        a[4] = pt_f2d(P.qomf * f4);
-        a[5] = pt_f2d(P.qomf * f5);
+        a[3] = P.qomf * f3;
+        a[4] = P.qomf * f4;
+        a[5] = P.qomf * f5;
+    }
+
+    /* The evaluation of the lane-per-particle machine; every FP64 <-> FP32
+     * conversion on the integer pipe.  The FP64 stage state s is not needed. */
+    static __device__ __forceinline__ void f(const PtRun &P, const double *, const double d[6],
+                                             const Origin &O, double a[6])
+    {
+        float df[6], af[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) df[c] = pt_d2f(d[c]);
+        f32(P, df, O, af);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) a[c] = pt_f2d(af[c]);
+    }
+
+    /* Eight lanes per particle (pt_coop.cuh): every lane rounds its own
+     * component of d; the FP32 evaluation is cheap next to one FP64 slot and
+     * runs on all lanes alike (their loads fall on the same addresses). */
+    static constexpr int kCoopRows = 0;
+    using CoopOrigin = Origin;
+    static __device__ __forceinline__ void coop_begin(const PtRun &P, const pt_sm::Group &Q, double si,
+                                                      Origin &O)
+    {
+        const double xn = fma(si, P.gsx[Q.ax], P.gox[Q.ax]);
+        const double fl = pt_floor(xn);
+        const float off = pt_d2f(xn - fl), u = pt_d2f(si);
+        const int32_t cell = pt_i32(fl);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            O.cell[i] = Q.get(cell, i);
+            O.off[i] = Q.get(off, i);
+            O.u[i] = Q.get(u, 3 + i);
+        }
+    }
+    static __device__ __forceinline__ double coop_f(const PtRun &P, const pt_sm::Group &Q, double *,
+                                                    double, double d, const Origin &O)
+    {
+        const float own = pt_d2f(d);
+        float df[6], af[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) df[c] = Q.get(own, c);
+        f32(P, df, O, af);
+        float r = af[0];
+#pragma unroll
+        for (int c = 1; c < 6; ++c) r = (Q.c == c) ? af[c] : r;
+        return pt_f2d(r);
+    }
+    static __device__ __forceinline__ double coop_face_cap(const PtRun &P, const pt_sm::Group &, double,
+                                                           const Origin &O, double h)
+    {
+        return pt_sm::pt_face_cap(P, O.off, O.u, h);
     }
 };
 
@@ -336,19 +383,38 @@ template <int METHOD, class EV, bool LEARN, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
 k_integrate_mixed(const PtRun P)
 {
-    pt_sm::run_machine<METHOD, EV, LEARN>(pt_sm::Members<false>{ P });
+    pt_sm::run_machine<METHOD, EV, LEARN, false, !LEARN>(pt_sm::Members<false>{ P });
+}
+
+template <int METHOD, class EV>
+__global__ void __launch_bounds__(128, 3) k_coop_mixed(const PtRun P, bool from_queue)
+{
+    pt_sm::run_coop<METHOD, EV>(pt_sm::Members<false>{ P }, from_queue);
+}
+
+template <int METHOD, class EV>
+__global__ void __launch_bounds__(128, 3) k_ensemble_coop_mixed(const PtRun *__restrict__ tab, int nmem,
+                                                                int64_t few)
+{
+    __shared__ PtRun sP[PT_ENS_MAX];
+    __shared__ int64_t sN[PT_ENS_MAX];
+    pt_sm::ens_load(tab, nmem, sP, sN);
+    const pt_sm::Members<true> MB{ sP, sN, nmem };
+    pt_sm::run_coop<METHOD, EV, true>(MB, MB.total() <= few);
 }
 
 /* Several runs (members: snapshots, tolerances, particle sets) in one
  * persistent launch; every lane drains the members' queues in table order. */
 template <int METHOD, class EV, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
-k_ensemble_mixed(const PtRun *__restrict__ tab, int nmem)
+k_ensemble_mixed(const PtRun *__restrict__ tab, int nmem, int64_t few)
 {
     __shared__ PtRun sP[PT_ENS_MAX];
     __shared__ int64_t sN[PT_ENS_MAX];
     pt_sm::ens_load(tab, nmem, sP, sN);
-    pt_sm::run_machine<METHOD, EV, false, true>(pt_sm::Members<true>{ sP, sN, nmem });
+    const pt_sm::Members<true> MB{ sP, sN, nmem };
+    if (MB.total() <= few) return;                 /* k_ensemble_coop_mixed takes the queue */
+    pt_sm::run_machine<METHOD, EV, false, true, true>(MB);
 }
 
 template <class EV>
@@ -388,7 +454,8 @@ cudaError_t launch_ens1(const PtRun *tab, int nmem, int block, int64_t ntot, cud
     const int smem = pt_sm::smem_bytes<METHOD>(block, false);
     return pt_sm::launch_persistent(k_ensemble_mixed<METHOD, EV, MINB>, block, smem,
                                     pt_sm::smem_bytes<METHOD>(PT_BLOCK_MAX, false), cache,
-                                    ntot, s, tab, nmem);
+                                    ntot, s, tab, nmem,
+                                    (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
 }
 
 template <int METHOD, class EV>
@@ -397,11 +464,18 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
 {
     if (ntot == 0) return cudaSuccess;          /* ntot < 0: configure only */
     if (!block) block = PT_BLOCK_DEFAULT;
+    cudaError_t e;
     switch (minb) {
-    case 2: return launch_ens1<METHOD, EV, 2>(tab, nmem, block, ntot, s);
-    case 4: return launch_ens1<METHOD, EV, 4>(tab, nmem, block, ntot, s);
-    default: return launch_ens1<METHOD, EV, 3>(tab, nmem, block, ntot, s);
+    case 2: e = launch_ens1<METHOD, EV, 2>(tab, nmem, block, ntot, s); break;
+    case 4: e = launch_ens1<METHOD, EV, 4>(tab, nmem, block, ntot, s); break;
+    default: e = launch_ens1<METHOD, EV, 3>(tab, nmem, block, ntot, s); break;
     }
+    /* how many particles are left is known on the device only: both kernels
+     * are launched, and the one that is not to take the queue finds nothing */
+    if (e == cudaSuccess && ntot > 0)
+        e = pt_sm::launch_coop<METHOD, EV>(k_ensemble_coop_mixed<METHOD, EV>, -1, s, tab, nmem,
+                                           (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
+    return e;
 }
 
 template <int METHOD, class EV, bool LEARN>
@@ -420,7 +494,11 @@ cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
     if (LEARNABLE && (P.mlp || P.rec)) return launch_v<METHOD, EV, LEARNABLE>(P, s);
-    return launch_v<METHOD, EV, false>(P, s);
+    const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+    cudaError_t e = few ? cudaSuccess : launch_v<METHOD, EV, false>(P, s);
+    if (e == cudaSuccess && (few || P.hand.ctl))
+        e = pt_sm::launch_coop<METHOD, EV>(k_coop_mixed<METHOD, EV>, few ? P.np : -1, s, P, few);
+    return e;
 }
 
 using F32_8 = EvalMixed<GatherF32<8>>;

@@ -43,3 +43,59 @@ def test_exact_bitwise_at_every_size(cuda, oracle_lib, method, with_j, near, siz
     assert np.array_equal(st.cpu().numpy(), sto)
     assert np.array_equal(c.cpu().numpy(), co)
     assert np.array_equal(s.cpu().numpy().view(np.int64), so.view(np.int64))
+
+
+@pytest.mark.parametrize("method,tol", [("rk5", 1e-8), ("dop853", 1e-8)])
+@pytest.mark.parametrize("prec,kw", [("fp64_fma", {}), ("fp64_fma", dict(face_steps=True)), ("fp32", {}),
+                                     ("fp32", dict(face_steps=True, noise_floor=True)),
+                                     ("bf16", dict(noise_floor=True))])
+@pytest.mark.parametrize("with_j", [False, True])
+def test_both_machines_give_the_same_bits(cuda, method, tol, prec, kw, with_j):
+    """A particle's result does not depend on how many others run with it: a
+    few of them alone (eight lanes throughout) against the same ones in a run
+    that starts on one lane each and hands over."""
+    torch = cuda
+    from particles_gb300 import Fields
+    few = 333
+    npart = 3 * PER_SM * torch.cuda.get_device_properties(0).multi_processor_count + 17
+    prob = small_problem(method, n=20, npart=npart, periods=0.1, seed=72, with_j=with_j, nsteps=7,
+                         gamma_range=(1.001, 50.0), tol=tol)
+    t = lambda a: torch.tensor(a, device="cuda")
+    f = Fields(*prob["fields"], precision=prec)
+    out = []
+    for n in (npart, few):
+        s, c = t(prob["state"][:n]), torch.zeros((n, 3), dtype=torch.int64, device="cuda")
+        st = torch.zeros(n, dtype=torch.int32, device="cuda")
+        f.run_device(method, prob["params"], t(prob["time"]), s, c, st, eta=1e-3 if with_j else 0.0, **kw)
+        assert f.run_check() == 0
+        out.append((s[:few].cpu(), c[:few].cpu(), st[:few].cpu()))
+    for a, b in zip(*out):
+        assert torch.equal(a.view(torch.int64) if a.is_floating_point() else a,
+                           b.view(torch.int64) if b.is_floating_point() else b)
+    # finished, with output rows (the last one's time may round past tmax)
+    assert (out[0][2] == 0).all() and (out[0][0][:, -2, 6] > 1.0).all()
+
+
+def test_ensemble_of_few_and_many(cuda, oracle_lib):
+    """An ensemble's windows go to one machine or the other by the particles
+    that are left; the members' bits stay the oracle's."""
+    torch = cuda
+    import oracle
+    from particles_gb300 import Ensemble, Fields
+    few = PER_SM * torch.cuda.get_device_properties(0).multi_processor_count
+    z = lambda shape, dt: torch.zeros(shape, dtype=dt, device="cuda")
+    for counts in ((40, 7), (few, 50)):
+        probs = [small_problem("dop853", n=12, npart=n, periods=0.05, seed=80 + k, nsteps=3,
+                               gamma_range=(1.001, 50.0)) for k, n in enumerate(counts)]
+        mem = [dict(fields=Fields(*p["fields"]), params=p["params"], time=torch.tensor(p["time"], device="cuda"),
+                    state=torch.tensor(p["state"], device="cuda"), cnt=z((n, 3), torch.int64),
+                    status=z(n, torch.int32), carry=z(128 * n, torch.uint8)) for p, n in zip(probs, counts)]
+        es = Ensemble("dop853", mem)
+        for stop in (0.3 * probs[0]["time"][-1], 0.6 * probs[0]["time"][-1], 0.0):
+            es.run(stop)
+        live, _ = es.counts()
+        assert es.check() == 0 and (live == 0).all()
+        for p, m in zip(probs, mem):
+            so, co, _ = oracle.integrate("dop853", p["params"], p["time"], *p["fields"], p["state"].copy())
+            assert np.array_equal(m["cnt"].cpu().numpy(), co)
+            assert np.array_equal(m["state"].cpu().numpy().view(np.int64), so.view(np.int64))
