@@ -66,80 +66,193 @@ __global__ void k_pack_f32(int32_t d0, int32_t d1, int32_t d2, int32_t nbx, int3
     }
 }
 
+/* Doubles in the order of their values as unsigned integers (-0 below +0):
+ * the high and the low word of the key, and its value again. */
+__device__ __forceinline__ uint32_t pt_key_hi(double x)
+{
+    const int32_t hi = __double2hiint(x);
+    return (uint32_t)hi ^ ((uint32_t)(hi >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ uint32_t pt_key_lo(double x)
+{
+    return (uint32_t)__double2loint(x) ^ (uint32_t)(__double2hiint(x) >> 31);
+}
+__device__ __forceinline__ double pt_key_value(uint32_t hi, uint32_t lo)
+{
+    const uint32_t s = (hi >> 31) ? 0u : 0xffffffffu;      /* negative: all bits inverted */
+    return __hiloint2double((int)(hi ^ (s | 0x80000000u)), (int)(lo ^ s));
+}
+
+/* The rarely needed FP64 quotient, out of line: inlined, parts of the division
+ * run ahead of the test that decides on it. */
+__noinline__ __device__ float pt_pack_quotient(double v, float off, float sc)
+{
+    return (float)((v - (double)off) / (double)sc);
+}
+
 /* Planar reference layout -> BF16 8^3 bricks with a one-node halo on the
  * high faces (9^3 records per brick; record (lx, ly, lz) of brick (bx, by,
- * bz) holds node ((8 bx + lx) mod d0, ...)), one block of 768 threads per
- * brick, one thread per record.  Per component the brick's offset is the
+ * bz) holds node ((8 bx + lx) mod d0, ...)), one block per brick.  Per component the brick's offset is the
  * midpoint and its scale the half-range of the component over the records a
  * stencil can reach (8 b + l <= d on every axis), both rounded to FP32; a
- * record stores q = (v - offset) / scale rounded to BF16 (|q| <= 1). */
+ * record stores q = (v - offset) / scale rounded to BF16 (|q| <= 1).
+ *
+ * The bound is HBM (with eta J 1.97 GB at 256^3, 0.29 ms); the FP64 pipe, at one
+ * instruction per 64 cycles and scheduler, must stay out of the way.  So the
+ * extremes are taken on integer keys, the high words first and the low words
+ * among the few values that share the extreme high word, and the quotient --
+ * FP64 division, rounded to FP32, rounded to BF16 -- is formed in FP32 from
+ * v split into two floats, offset and 1/scale: within 7 FP32 ulps of the twice
+ * rounded one, so their BF16 roundings agree unless a BF16 midpoint lies
+ * within 8 ulps, and then (also where v nearly cancels the offset, or leaves
+ * the FP32 normal range) the division decides.  256^3: 0.75 ms (0.45 without J);
+ * with FP64 reductions and divisions it was 9.95 (6.91). */
+template <int NV> struct PackShape {
+    /* records per thread, blocks per SM; 1 x 2, 2 x 3, 3 x 3, 4 x 4 measured 944,
+     * 748, 764, 868 us with J and 1 x 2, 2 x 3, 3 x 3, 3 x 4, 4 x 4 601, 535,
+     * 492, 452, 462 us without (256^3) */
+    static constexpr int kRecords = NV == 9 ? 2 : 3, kBlocks = NV == 9 ? 3 : 4;
+    static constexpr int kThreads = 768 / kRecords;
+};
 template <int NV>
-__global__ void __launch_bounds__(768) k_pack_bricks16(int32_t d0, int32_t d1, int32_t d2,
-                                                       int32_t nbx, int32_t nby,
-                                                       const double *__restrict__ uu,
-                                                       const double *__restrict__ bb,
-                                                       const double *__restrict__ jj,
-                                                       uint4 *__restrict__ rec,
-                                                       float *__restrict__ bscale)
+__global__ void __launch_bounds__(PackShape<NV>::kThreads, PackShape<NV>::kBlocks) k_pack_bricks16(int32_t d0, int32_t d1, int32_t d2,
+                                                          int32_t nbx, int32_t nby,
+                                                          const double *__restrict__ uu,
+                                                          const double *__restrict__ bb,
+                                                          const double *__restrict__ jj,
+                                                          uint4 *__restrict__ rec,
+                                                          float *__restrict__ bscale)
 {
-    constexpr int NC16 = (NV == 9) ? 16 : 8, NS = (NV == 9) ? 20 : 12;
-    __shared__ double smin[24][NV], smax[24][NV];
-    __shared__ float soff[NV], ssc[NV];
+    constexpr int NC16 = (NV == 9) ? 16 : 8, NS = (NV == 9) ? 20 : 12, NR = PackShape<NV>::kRecords;
+    constexpr int NT = PackShape<NV>::kThreads, NU = 2 * NV;   /* threads; half components */
+    __shared__ uint32_t keys[NV][NR * NT];                  /* high words */
+    __shared__ uint32_t umin[NU], umax[NU], lmin[NV], lmax[NV];
+    __shared__ float foff[NV], fsc[NV], srs[NV];
     const int64_t b = blockIdx.x;
     const int bx = (int)(b % nbx), by = (int)((b / nbx) % nby), bz = (int)(b / ((int64_t)nbx * nby));
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int lx = t % 9, ly = (t / 9) % 9, lz = t / 81;
-    const int gi = bx * 8 + lx, gj = by * 8 + ly, gk = bz * 8 + lz;
-    const bool slot = t < 729;
-    const bool reach = slot && gi <= d0 && gj <= d1 && gk <= d2;
-    const int i = gi % d0, j = gj % d1, k = gk % d2;
+    const int lane = threadIdx.x & 31;
     const int64_t nn = (int64_t)d0 * d1 * d2;
-    const int64_t g = i + (int64_t)d0 * (j + (int64_t)d1 * k);
-    double v[NV];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        v[c] = reach ? uu[g + c * nn] : 0.0;
-        v[3 + c] = reach ? bb[g + c * nn] : 0.0;
-        if (NV == 9) v[(6 + c) % NV] = reach ? jj[g + c * nn] : 0.0;
+    const double *const src[3] = { uu, bb, jj };
+    if (threadIdx.x < NV) {
+        lmin[threadIdx.x] = 0xffffffffu;
+        lmax[threadIdx.x] = 0u;
     }
+    /* Node of record t, or -1 if no stencil reaches it (8 b < d, so within
+     * reach a coordinate is the extent itself at most). */
+    auto node = [&](int t) -> int64_t {
+        const int gi = bx * 8 + t % 9, gj = by * 8 + (t / 9) % 9, gk = bz * 8 + t / 81;
+        if (t >= 729 || gi > d0 || gj > d1 || gk > d2) return -1;
+        const int i = gi == d0 ? 0 : gi, j = gj == d1 ? 0 : gj, k = gk == d2 ? 0 : gk;
+        return i + (int64_t)d0 * (j + (int64_t)d1 * k);
+    };
+    double v[NR][NV];
+    bool reach[NR];
+    const int64_t first = node(0);
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        double mn = reach ? v[c] : INFINITY, mx = reach ? v[c] : -INFINITY;
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        }
-        if (lane == 0) { smin[warp][c] = mn; smax[warp][c] = mx; }
+    for (int n = 0; n < NR; ++n) {
+        const int t = threadIdx.x + NT * n;
+        int64_t g = node(t);
+        reach[n] = g >= 0;
+        if (!reach[n]) g = first;             /* stands in, so the extremes need no mask */
+#pragma unroll
+        for (int c = 0; c < NV; ++c) v[n][c] = __ldg(src[c / 3] + g + (c % 3) * nn);
+#pragma unroll
+        for (int c = 0; c < NV; ++c) keys[c][t] = pt_key_hi(v[n][c]);
     }
     __syncthreads();
-    if (t < NV) {
-        double mn = smin[0][t], mx = smax[0][t];
-        for (int w = 1; w < 24; ++w) { mn = fmin(mn, smin[w][t]); mx = fmax(mx, smax[w][t]); }
+    /* a warp per half component: 12 keys per lane, then one warp reduction */
+    for (int u = threadIdx.x >> 5; u < NU; u += NT / 32) {
+        const uint32_t *k = &keys[u >> 1][(u & 1) * (NR * NT / 2) + lane];
+        uint32_t mn = k[0], mx = k[0];
+#pragma unroll
+        for (int i = 32; i < NR * NT / 2; i += 32) {
+            mn = min(mn, k[i]);
+            mx = max(mx, k[i]);
+        }
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0) {
+            umin[u] = mn;
+            umax[u] = mx;
+        }
+    }
+    __syncthreads();
+    /* low words among the few values with an extreme high word */
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+        const uint32_t mn = min(umin[2 * c], umin[2 * c + 1]), mx = max(umax[2 * c], umax[2 * c + 1]);
+#pragma unroll
+        for (int n = 0; n < NR; ++n) {
+            const uint32_t k = pt_key_hi(v[n][c]);
+            if (k == mn) atomicMin(&lmin[c], pt_key_lo(v[n][c]));
+            if (k == mx) atomicMax(&lmax[c], pt_key_lo(v[n][c]));
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        const int c = threadIdx.x;
+        double mn = pt_key_value(min(umin[2 * c], umin[2 * c + 1]), lmin[c]);
+        double mx = pt_key_value(max(umax[2 * c], umax[2 * c + 1]), lmax[c]);
+        if (mn != mn || mx != mx) {      /* NaN values do not take part in the extremes */
+            mn = INFINITY;
+            mx = -INFINITY;
+            for (int t = 0; t < 729; ++t) {
+                const int64_t g = node(t);
+                const double x = g >= 0 ? src[c / 3][g + (c % 3) * nn] : NAN;
+                mn = fmin(mn, x);
+                mx = fmax(mx, x);
+            }
+        }
         const float off = (float)(0.5 * (mn + mx));
         float sc = (float)(0.5 * (mx - mn));
         if (!(sc > 0.0f)) sc = 1.0f;
-        soff[t] = off;
-        ssc[t] = sc;
-        bscale[b * NS + 2 * t] = off;
-        bscale[b * NS + 2 * t + 1] = sc;
-    } else if (t >= 2 * NV && t < NS) {
-        bscale[b * NS + t] = 0.0f;
+        foff[c] = off;
+        fsc[c] = sc;
+        /* 0 turns the FP32 quotient off: 1/sc or v - off may leave its normal range */
+        srs[c] = (sc > 1.0e-15f && sc < 1.0e15f) ? 1.0f / sc : 0.0f;
+        bscale[b * NS + 2 * c] = off;
+        bscale[b * NS + 2 * c + 1] = sc;
+    } else if (threadIdx.x >= 2 * NV && threadIdx.x < NS) {
+        bscale[b * NS + threadIdx.x] = 0.0f;
     }
     __syncthreads();
-    if (!slot) return;
-    unsigned short q[NC16];
 #pragma unroll
-    for (int c = 0; c < NC16; ++c) q[c] = 0;
+    for (int n = 0; n < NR; ++n) {
+        const int t = threadIdx.x + NT * n;
+        float x[NC16];
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        const float x = reach ? (float)((v[c] - (double)soff[c]) / (double)ssc[c]) : 0.0f;
-        q[c] = __bfloat16_as_ushort(__float2bfloat16_rn(x));
+        for (int c = 0; c < NC16; ++c) x[c] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+            /* v = vh + vl: its first 24 significant bits and the next 23 of the
+             * rest, as floats (exponents 2^-63 .. 2^127, rebiased by one bit flip) */
+            const uint32_t hi = (uint32_t)__double2hiint(v[n][c]), lo = (uint32_t)__double2loint(v[n][c]);
+            const uint32_t sg = hi & 0x80000000u;
+            const uint32_t f = ((__funnelshift_l(lo, hi, 3) & 0x7fffffffu) ^ 0x40000000u);
+            const uint32_t e2 = (f & 0x7f800000u) - (23u << 23);
+            const float vl = __uint_as_float(e2 | sg | ((lo >> 6) & 0x7fffffu)) - __uint_as_float(e2 | sg);
+            const float vh = __uint_as_float(f | sg);
+            const float d = (vh - foff[c]) + vl;
+            x[c] = d * srs[c];
+            const uint32_t xb = __float_as_uint(x[c]);
+            const bool tie = (xb & 0xffffu) - 0x7ff8u <= 16u;
+            const bool range = (hi & 0x7fffffffu) - 0x3c000000u < 0x47e00000u - 0x3c000000u;
+            if ((tie | !range | (fabsf(d) < 4.8e-7f * fabsf(vh)) | (srs[c] == 0.0f)) && reach[n])
+                x[c] = pt_pack_quotient(v[n][c], foff[c], fsc[c]);
+            if (!reach[n]) x[c] = 0.0f;
+        }
+        if (t < 729) {
+            uint32_t q[NC16 / 2];
+#pragma unroll
+            for (int w = 0; w < NC16 / 2; ++w) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * w], x[2 * w + 1]);
+                q[w] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+            uint4 *o = rec + (b * 729 + t) * (NC16 / 8);
+#pragma unroll
+            for (int w = 0; w < NC16 / 8; ++w) o[w] = make_uint4(q[4 * w], q[4 * w + 1], q[4 * w + 2], q[4 * w + 3]);
+        }
     }
-    uint4 *o = rec + (b * 729 + t) * (NC16 / 8);
-#pragma unroll
-    for (int w = 0; w < NC16 / 8; ++w)
-        o[w] = make_uint4(q[8 * w] | ((uint32_t)q[8 * w + 1] << 16), q[8 * w + 2] | ((uint32_t)q[8 * w + 3] << 16),
-                          q[8 * w + 4] | ((uint32_t)q[8 * w + 5] << 16), q[8 * w + 6] | ((uint32_t)q[8 * w + 7] << 16));
 }
 
 static bool dims_ok(const int32_t dm[3])
@@ -213,10 +326,10 @@ static int fields_create_impl(const int32_t dm[3], const double *uu, const doubl
         if (blocks > 65536) blocks = 65536;
         const int64_t nbk = (int64_t)f->nb[0] * f->nb[1] * f->nb[2];
         if (precision == PT_PREC_BF16 && f->has_j)
-            k_pack_bricks16<9><<<(unsigned)nbk, 768, 0, stream>>>(dm[0], dm[1], dm[2], f->nb[0], f->nb[1],
+            k_pack_bricks16<9><<<(unsigned)nbk, PackShape<9>::kThreads, 0, stream>>>(dm[0], dm[1], dm[2], f->nb[0], f->nb[1],
                                                                   d_uu, d_bb, d_jj, f->rec16, f->bscale);
         else if (precision == PT_PREC_BF16)
-            k_pack_bricks16<6><<<(unsigned)nbk, 768, 0, stream>>>(dm[0], dm[1], dm[2], f->nb[0], f->nb[1],
+            k_pack_bricks16<6><<<(unsigned)nbk, PackShape<6>::kThreads, 0, stream>>>(dm[0], dm[1], dm[2], f->nb[0], f->nb[1],
                                                                   d_uu, d_bb, d_jj, f->rec16, f->bscale);
         else if (precision == PT_PREC_FP32)
             k_pack_f32<<<(int)((nbk * 512 + 255) / 256 < 65536 ? (nbk * 512 + 255) / 256 : 65536), 256, 0,
