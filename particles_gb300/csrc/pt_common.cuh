@@ -179,37 +179,23 @@ __device__ __forceinline__ double pt_max(double a, double b) { return (b > a) ? 
 __device__ __forceinline__ double pt_min(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double pt_nanmax(double m, double q) { return (q > m || q != q) ? q : m; }
 
-/* floor(x) for doubles on the integer pipe.  GB300 runs 2 FP64 operations
- * per cycle per SM and the FP64 rounding and conversion instructions share
- * that pipe, while integer operations run at 64 per cycle; floor is exact, so
- * clearing the fraction bits (after a carry into the integer bits for a
- * negative non-integer) gives the same value as the FP64 instruction,
- * including -0.0, +-inf and NaN. */
-__device__ __forceinline__ double pt_floor(double x)
+/* Comparisons on the integer pipe (an FP64 comparison takes an FP64 slot: with
+ * them, the floors' hidden ones and the unused FP64 stage state gone, 262,144
+ * particles RK5 FP32 25.6 -> 23.2 ms, DOP853 FP32 43.0 -> 39.8, RK5 exact
+ * 57.5 -> 55.2).
+ * pt_isnan for any x; pt_le: a <= b and pt_gt: a > b for b >= +0 and any a but NaN;
+ * pt_max_pos: pt_max of magnitudes (a NaN may win where pt_max keeps a number). */
+__device__ __forceinline__ bool pt_isnan(double x)
 {
-    const long long b = __double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ff) - 1023;
-    if (e >= 52) return x;                                  /* integral, inf or NaN */
-    if (e < 0)                                              /* |x| < 1 */
-        return (b < 0) ? ((b & 0x7fffffffffffffffLL) ? -1.0 : x) : __longlong_as_double(0LL);
-    const long long frac = 0x000fffffffffffffLL >> e;
-    if ((b & frac) == 0) return x;
-    return __longlong_as_double(((b < 0) ? b + frac : b) & ~frac);
+    const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    return h > 0x7ff00000u || (h == 0x7ff00000u && __double2loint(x) != 0);
 }
-
-/* (int32_t)q for an integral double q on the integer pipe, saturating at
- * the int32 range like the hardware conversion (NaN -> 0). */
-__device__ __forceinline__ int32_t pt_i32(double q)
+__device__ __forceinline__ bool pt_le(double a, double b)
 {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(q);
-    const int e = (int)((b >> 52) & 0x7ff) - 1023;
-    const bool neg = (b >> 63) != 0;
-    if (e == 1024 && (b & 0x000fffffffffffffULL)) return 0;            /* NaN */
-    if (e < 0) return 0;
-    if (e > 30) return neg ? (int32_t)0x80000000u : 0x7fffffff;
-    const int32_t v = (int32_t)(((b & 0x000fffffffffffffULL) | (1ULL << 52)) >> (52 - e));
-    return neg ? -v : v;
+    return __double_as_longlong(a) <= __double_as_longlong(b);
 }
+__device__ __forceinline__ bool pt_gt(double a, double b) { return !pt_le(a, b); }
+__device__ __forceinline__ double pt_max_pos(double a, double b) { return pt_le(b, a) ? a : b; }
 
 /* floor(xp) as a 0-based node index; dm (only reachable when x - floor(x)
  * rounds up to 1 for a tiny negative x, where the reference indexes past the
@@ -217,10 +203,11 @@ __device__ __forceinline__ int32_t pt_i32(double q)
  * integral double (a floor), read off its bits on the integer pipe. */
 __device__ __forceinline__ int32_t pt_node_index(double q, int32_t d)
 {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(q);
-    const int e = (int)((b >> 52) & 0x7ff) - 1023;
-    if ((b >> 63) || e < 0 || e > 30) return 0;            /* negative, < 1, huge, inf, NaN */
-    const int32_t v = (int32_t)(((b & 0x000fffffffffffffULL) | (1ULL << 52)) >> (52 - e));
+    const uint32_t hi = (uint32_t)__double2hiint(q), lo = (uint32_t)__double2loint(q);
+    const uint32_t e = (hi >> 20) - 1023u;                 /* with the sign bit: > 30 if negative */
+    if (e > 30u) return 0;                                 /* negative, < 1, huge, inf, NaN */
+    const uint32_t m = (hi & 0xfffffu) | 0x100000u;
+    const int32_t v = (int32_t)(e < 20u ? m >> (20u - e) : __funnelshift_l(lo, m, e - 20u));
     return v < d ? v : 0;
 }
 
@@ -305,8 +292,9 @@ __device__ __forceinline__ int32_t pt_attempt_guard(double t, double dt, int64_t
                                                     int64_t max_steps)
 {
     if (max_steps > 0 && attempts >= max_steps) return PT_ST_STEP_LIMIT;
-    if (dt != dt) return PT_ST_NONFINITE;
-    if (!(dt > 0.0) || t + dt == t) return PT_ST_DT_UNDERFLOW;
+    if (pt_isnan(dt)) return PT_ST_NONFINITE;
+    /* dt > 0, and t >= 0 moves: on the bits */
+    if (pt_le(dt, 0.0) || __double_as_longlong(t + dt) == __double_as_longlong(t)) return PT_ST_DT_UNDERFLOW;
     return PT_GO;
 }
 

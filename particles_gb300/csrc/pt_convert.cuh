@@ -18,44 +18,34 @@
 
 #include <stdint.h>
 
-/* double -> float, round to nearest even. */
+/* double -> float outside the float normal range: zero, infinity, NaN. */
+__device__ __noinline__ inline float pt_d2f_special(uint32_t hi, uint32_t lo)
+{
+    const uint32_t sign = hi & 0x80000000u, e = (hi >> 20) & 0x7ffu;
+    if (e == 0x7ffu && ((hi & 0xfffffu) | lo)) return __uint_as_float(sign | 0x7fc00000u);
+    return __uint_as_float(e < 897u ? sign : sign | 0x7f800000u);
+}
+
+/* double -> float, round to nearest even: in the float normal range the
+ * exponent is rebiased by dropping its two top bits and flipping the next
+ * (biased 897..1150 -> 1..254), and the 29 dropped bits decide the rounding
+ * (whose carry may bump the exponent). */
 __device__ __forceinline__ float pt_d2f(double x)
 {
-    const uint64_t b = (uint64_t)__double_as_longlong(x);
-    const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
-    const uint32_t sign = hi & 0x80000000u;
-    const int e = (int)((hi >> 20) & 0x7ffu);
-    if (e == 0x7ff)                                   /* inf or NaN */
-        return __uint_as_float(sign | 0x7f800000u | ((hi & 0xfffffu) | lo ? 0x400000u : 0u));
-    const int ef = e - 1023 + 127;
-    if (ef <= 0) return __uint_as_float(sign);         /* below float normals: signed zero */
-    if (ef >= 255) return __uint_as_float(sign | 0x7f800000u);
-    const uint32_t m = ((hi & 0xfffffu) << 3) | (lo >> 29);   /* top 23 mantissa bits */
-    const uint32_t rest = lo & 0x1fffffffu;                    /* the 29 dropped bits */
-    uint32_t f = sign | ((uint32_t)ef << 23) | m;
-    f += (rest > 0x10000000u) | ((rest == 0x10000000u) & (m & 1u));  /* carry may bump the exponent */
-    return __uint_as_float(f);
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    if ((hi & 0x7fffffffu) - 0x38100000u >= 0x47f00000u - 0x38100000u) return pt_d2f_special(hi, lo);
+    const uint32_t f = ((__funnelshift_l(lo, hi, 3) & 0x7fffffffu) ^ 0x40000000u) | (hi & 0x80000000u);
+    return __uint_as_float(f + ((lo & 0x1fffffffu) + (f & 1u) > 0x10000000u ? 1u : 0u));
 }
 
 /* float -> double, exact (float subnormals flush to zero). */
 __device__ __forceinline__ double pt_f2d(float f)
 {
-    const uint32_t b = __float_as_uint(f);
-    const uint32_t sign = b & 0x80000000u;
-    const uint32_t e = (b >> 23) & 0xffu;
-    const uint32_t m = b & 0x7fffffu;
-    uint32_t hi, lo;
-    if (e == 0) {
-        hi = sign;
-        lo = 0u;
-    } else if (e == 0xffu) {
-        hi = sign | 0x7ff00000u | (m >> 3);
-        lo = m << 29;
-    } else {
-        hi = sign | ((e + 896u) << 20) | (m >> 3);
-        lo = m << 29;
-    }
-    return __hiloint2double((int)hi, (int)lo);
+    const uint32_t b = __float_as_uint(f), a = b & 0x7fffffffu;
+    uint32_t hi = (a >> 3) + 0x38000000u, lo = b << 29;
+    if (a >= 0x7f800000u) hi += 0x38000000u;               /* inf, NaN */
+    if (a < 0x00800000u) hi = lo = 0u;
+    return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
 }
 
 #endif /* PT_CONVERT_CUH */

@@ -195,7 +195,7 @@ __device__ __forceinline__ void coop_step(double h, double k, double si, double 
     s = si + x;
 #else
     d = __dmul_rn(h, k);
-    s = DELTA ? __dadd_rn(si, d) : fma(h, k, si);
+    s = DELTA ? __dadd_rn(si, d) : fma(h, k, si);   /* (unused, and dropped, in DELTA stages) */
 #endif
 }
 
@@ -219,7 +219,6 @@ __device__ __forceinline__ void coop_stage(int j, const KOwn &K, double si, doub
             double acc = S.a[0] * K(S.r[0]);
             for (int i = 1; i < S.n; ++i) acc = acc + S.a[i] * K(S.r[i]);
             dl = acc;
-            ss = si + acc;
         } else {
             PtR acc = si;
             for (int i = 0; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i]);
@@ -235,7 +234,7 @@ __device__ __forceinline__ double coop_group_max(const Group &G, double v)
     const int b = G.c < 3 ? 0 : 3;
     const double a = fabs(v);
     const double v0 = G.get(a, b), v1 = G.get(a, b + 1), v2 = G.get(a, b + 2);
-    return pt_max(v0, pt_max(v1, v2));
+    return pt_max_pos(v0, pt_max_pos(v1, v2));
 }
 #endif
 
@@ -249,7 +248,7 @@ __device__ __forceinline__ double coop_finish(const PtRun &P, const Group &G, co
         const PtR k4 = PtR(B01) * K(0) + PtR(B06) * K(5) + PtR(B07) * K(6) + PtR(B08) * K(7)
                      + PtR(B09) * K(8) + PtR(B10) * K(9) + PtR(B11) * K(1) + PtR(B12) * K(2);
         coop_step<DELTA>(dt, k4, si, sf, dsf);
-        double sr = PtR(P.atol) + PtR(P.rtol) * pt_max(fabs(si), fabs(sf));
+        double sr = PtR(P.atol) + PtR(P.rtol) * pt_max_pos(fabs(si), fabs(sf));
         const PtR e3 = k4 - PtR(BH1) * K(0) - PtR(BH2) * K(8) - PtR(BH3) * K(2);
         const PtR e5 = PtR(ER01) * K(0) + PtR(ER06) * K(5) + PtR(ER07) * K(6) + PtR(ER08) * K(7)
                      + PtR(ER09) * K(8) + PtR(ER10) * K(9) + PtR(ER11) * K(1) + PtR(ER12) * K(2);
@@ -278,9 +277,9 @@ __device__ __forceinline__ double coop_finish(const PtRun &P, const Group &G, co
         const double deno = err5 + 1.0e-02 * err3;
 #ifdef PT_EXACT
         const double num = PtR(fabs(dt)) * err5;
-        return num / sqrt((deno <= 0.0) ? 6.0 : (double)(PtR(6.0) * deno));
+        return num / sqrt(pt_le(deno, 0.0) ? 6.0 : (double)(PtR(6.0) * deno));
 #else
-        if (!(deno > 1.0e-300))
+        if (pt_le(deno, 1.0e-300))
             return (deno <= 0.0) ? fabs(dt) * err5 * 0.40824829046386307
                                  : fabs(dt) * err5 / sqrt(6.0 * deno);
         return fabs(dt) * err5 * pt_rsqrt(6.0 * deno);
@@ -346,10 +345,10 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
         if (j == 0) {
             if (active) {
                 q = coop_finish<METHOD, EV::kDelta>(PT_Q, G, K, si, L.dt, pt, dl);
-                if (q != q) {
+                if (pt_isnan(q)) {
                     coop_close<METHOD>(PT_Q, G, K, L, si, PT_ST_NONFINITE);
                     active = false;
-                } else if (q <= 1.0) {
+                } else if (pt_le(q, 1.0)) {
                     mode = M_ACCEPT;
                     need = true;
                 } else {

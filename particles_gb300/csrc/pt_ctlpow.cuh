@@ -26,8 +26,11 @@ __device__ __forceinline__ double pt_ctl_pow(double q, double y)
 #ifdef PT_EXACT
     return pt_det_pow(q, y);
 #else
-    const int n = (y == -0.2) ? 5 : (y == -0.25) ? 4 : (y == -0.125) ? 8 : 0;
-    if (n == 0 || !(q > 1e-30 && q < 1e30)) return pt_det_pow(q, y);
+    const long long yb = __double_as_longlong(y);
+    const int n = (yb == __double_as_longlong(-0.2)) ? 5 : (yb == __double_as_longlong(-0.25)) ? 4
+                : (yb == __double_as_longlong(-0.125)) ? 8 : 0;
+    if (n == 0 || pt_le(q, 1e-30) || !(__double_as_longlong(q) < __double_as_longlong(1e30)))
+        return pt_det_pow(q, y);
     const float inv = (n == 5) ? 0.2f : (n == 4) ? 0.25f : 0.125f;
     const double invd = (n == 5) ? 0.2 : (n == 4) ? 0.25 : 0.125;
     double x = pt_f2d(exp2f(-inv * __log2f(pt_d2f(q))));

@@ -89,6 +89,48 @@ PT_DM_FN double pt_dsub(double a, double b)
 #endif
 }
 
+#if defined(__CUDACC__)
+/* floor(x) for doubles on the integer pipe, in 32-bit words.  The FP64
+ * rounding, conversion and comparison instructions take the FP64 pipe's slots;
+ * floor is exact, so clearing the fraction bits (after a carry into the integer
+ * bits for a negative non-integer) gives the FP64 instruction's value,
+ * including -0.0, +-inf and NaN.  (On 64-bit words the compiler turns the
+ * tests of the fraction back into FP64 comparisons.) */
+__device__ __forceinline__ double pt_floor(double x)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
+    if (e >= 20) {
+        if (e >= 52) return x;                              /* integral, inf or NaN */
+        const long long b = __double_as_longlong(x), frac = (long long)(0xffffffffu >> (e - 20));
+        return __longlong_as_double(((b < 0) ? b + frac : b) & ~frac);
+    }
+    const uint32_t neg = hi >> 31;
+    const uint32_t mask = 0xfffffu >> (e & 31);             /* fraction bits of hi when e >= 0 */
+    const uint32_t up = (neg && ((hi & mask) | lo)) ? mask + 1u : 0u;
+    uint32_t r = (hi + up) & ~mask;
+    if (e < 0) r = neg ? (((hi << 1) | lo) ? 0xbff00000u : 0x80000000u) : 0u;   /* |x| < 1 */
+    return __hiloint2double((int)r, 0);
+}
+
+/* (int32_t)q for an integral double q on the integer pipe, saturating at
+ * the int32 range like the hardware conversion (NaN -> 0). */
+__device__ __forceinline__ int32_t pt_i32(double q)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(q), lo = (uint32_t)__double2loint(q);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
+    const bool neg = (hi >> 31) != 0;
+    if (e > 30) {
+        if (e == 1024 && ((hi & 0xfffffu) | lo)) return 0;                 /* NaN */
+        return neg ? (int32_t)0x80000000u : 0x7fffffff;
+    }
+    if (e < 0) return 0;
+    const uint32_t m = (hi & 0xfffffu) | 0x100000u;
+    const int32_t v = (int32_t)(e < 20 ? m >> (20 - e) : __funnelshift_l(lo, m, e - 20));
+    return neg ? -v : v;
+}
+#endif
+
 PT_DM_FN int64_t pt_dbits(double x)
 {
 #if defined(__CUDA_ARCH__)
@@ -136,7 +178,7 @@ PT_DM_FN double pt_det_log(double x)
     }
     e -= 1023;
     double mnt = pt_dfrom((bits & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
-    if (mnt > PT_SQRT2) {               /* keep m in [sqrt(1/2), sqrt(2)] */
+    if (pt_dbits(mnt) > 0x3ff6a09e667f3bcdLL) {   /* m > sqrt(2): keep m in [sqrt(1/2), sqrt(2)] */
         mnt = pt_dmul(mnt, 0.5);        /* exact */
         e += 1;
     }
@@ -162,10 +204,16 @@ PT_DM_FN double pt_det_log(double x)
 /* e^z for finite or infinite z. */
 PT_DM_FN double pt_det_exp(double z)
 {
-    if (z != z) return z;
-    if (z > 709.782712893384) return pt_dfrom(0x7ff0000000000000LL);
-    if (z < -745.1332191019412) return 0.0;
+    if (((pt_dbits(z) >> 52) & 0x7ff) >= 1023 + 9) {     /* |z| >= 512 or NaN */
+        if (z != z) return z;
+        if (z > 709.782712893384) return pt_dfrom(0x7ff0000000000000LL);
+        if (z < -745.1332191019412) return 0.0;
+    }
+#if defined(__CUDA_ARCH__)
+    double kf = pt_floor(pt_dadd(pt_dmul(z, PT_INV_LN2), 0.5));
+#else
     double kf = floor(pt_dadd(pt_dmul(z, PT_INV_LN2), 0.5));
+#endif
     double r  = pt_dsub(pt_dsub(z, pt_dmul(kf, PT_LN2_HI)), pt_dmul(kf, PT_LN2_LO));
     /* Taylor series of e^r to r^13, Horner form with 1/n! coefficients. */
     double p = 1.0 / 6227020800.0;                       /* 1/13! */
@@ -182,7 +230,11 @@ PT_DM_FN double pt_det_exp(double z)
     p = pt_dadd(pt_dmul(p, r), 0.5);                    /* 1/2!  */
     p = pt_dadd(pt_dmul(p, r), 1.0);
     p = pt_dadd(pt_dmul(p, r), 1.0);
+#if defined(__CUDA_ARCH__)
+    int k = pt_i32(kf);
+#else
     int k = (int)kf;
+#endif
     if (k > 1023) return pt_dmul(pt_dmul(p, pt_pow2i(1023)), pt_pow2i(k - 1023));
     if (k < -1021) return pt_dmul(pt_dmul(p, pt_pow2i(k + 1000)), pt_pow2i(-1000));
     return pt_dmul(p, pt_pow2i(k));
@@ -192,12 +244,18 @@ PT_DM_FN double pt_det_exp(double z)
  * x < 0 returns NaN (no integer-exponent special case is needed here). */
 PT_DM_FN double pt_det_pow(double x, double y)
 {
-    if (y == 0.0) return 1.0;
-    if (x != x || y != y) return x + y;
-    if (x == 1.0) return 1.0;
-    if (x < 0.0) return pt_dfrom(0x7ff8000000000000LL);
-    if (x == 0.0) return (y < 0.0) ? pt_dfrom(0x7ff0000000000000LL) : 0.0;
-    if (x > 1.7976931348623157e308) return (y < 0.0) ? 0.0 : x;
+    /* the special cases behind one integer test: x finite, > 0 and not 1, y
+     * finite and not 0 need none of them */
+    const uint64_t bx = (uint64_t)pt_dbits(x), by = (uint64_t)pt_dbits(y) << 1;
+    if (bx - 1 >= 0x7fefffffffffffffULL || bx == 0x3ff0000000000000ULL ||
+        by - 1 >= 0xffdfffffffffffffULL) {
+        if (y == 0.0) return 1.0;
+        if (x != x || y != y) return x + y;
+        if (x == 1.0) return 1.0;
+        if (x < 0.0) return pt_dfrom(0x7ff8000000000000LL);
+        if (x == 0.0) return (y < 0.0) ? pt_dfrom(0x7ff0000000000000LL) : 0.0;
+        if (x > 1.7976931348623157e308) return (y < 0.0) ? 0.0 : x;
+    }
     return pt_det_exp(pt_dmul(y, pt_det_log(x)));
 }
 

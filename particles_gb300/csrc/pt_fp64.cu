@@ -78,6 +78,13 @@ struct EvalF64 {
     static constexpr bool kDelta = false;
     struct Origin {};
     static __device__ __forceinline__ void begin(const PtRun &, const double *, Origin &) {}
+#ifndef PT_EXACT
+    static __device__ __forceinline__ double face_cap(const PtRun &P, const double si[6], const Origin &,
+                                                      double h)
+    {
+        return pt_sm::pt_face_cap(P, si, h);
+    }
+#endif
     static __device__ __forceinline__ void feature_cell(const PtRun &P, const double si[6],
                                                         const Origin &, int32_t l[3], int32_t r[3],
                                                         float xd[3])

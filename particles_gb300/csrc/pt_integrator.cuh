@@ -219,7 +219,7 @@ __device__ __forceinline__ void lane_hand(double *r, const KRows &K, const Lane 
 /* Status before an attempt: PT_GO = go on, else the particle closes. */
 __device__ __forceinline__ int32_t lane_check(const PtRun &P, const Lane &L, uint64_t t_start)
 {
-    if (!(L.t < P.tend)) return (L.t >= P.tmx) ? PT_ST_DONE : PT_ST_RUNNING;
+    if (pt_le(P.tend, L.t)) return pt_le(P.tmx, L.t) ? PT_ST_DONE : PT_ST_RUNNING;   /* t >= 0 */
     const int32_t g = pt_attempt_guard(L.t, L.dt, L.c0, P.max_steps);
     if (g != PT_GO) return g;
     if (P.budget_ns && pt_globaltimer() - t_start > P.budget_ns) return PT_ST_TIMEOUT;
@@ -293,7 +293,8 @@ __device__ __forceinline__ bool escaped_x(const PtRun &P, double x)
 /* Stage state of slot j (1..SLOTS-1) in the reference's operand order, and
  * its increment d = s - si.  DOP853 forms s = si + (dt * sum) (:368-415), so
  * the increment is exact and free; RK5 sums from si (:132-135), so with
- * DELTA the increment is summed first (mixed precision only). */
+ * DELTA the increment is summed first.  DELTA (mixed precision, whose
+ * evaluation needs the increment alone) leaves the state itself out. */
 template <int METHOD, bool DELTA>
 __device__ __forceinline__ void stage_state(int j, const KRows &K, const double si[6], double dt,
                                             double ss[6], double dl[6])
@@ -303,7 +304,7 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
         if (j == 1) {                                           /* :368 */
             const PtR h = PtR(dt) * S.a[0];
 #pragma unroll
-            for (int c = 0; c < 6; ++c) { const PtR d = h * K(0, c); dl[c] = d; ss[c] = si[c] + d; }
+            for (int c = 0; c < 6; ++c) { const PtR d = h * K(0, c); dl[c] = d; if (!DELTA) ss[c] = si[c] + d; }
         } else {                                                /* :371-415 */
 #if defined(PT_EXACT) && PT_SMUL_STAGE
             /* the coefficient products on the integer pipes (pt_smul_raw:
@@ -316,7 +317,7 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
                 for (int i = 1; i < S.n; ++i) acc = acc + pt_smul_raw(S.a[i], K(S.r[i], c), ok);
                 const PtR d = dt * acc;
                 dl[c] = d;
-                ss[c] = si[c] + d;
+                if (!DELTA) ss[c] = si[c] + d;
             }
             if (!ok)
 #endif
@@ -326,7 +327,7 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
                 for (int i = 1; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i], c);
                 const PtR d = dt * acc;
                 dl[c] = d;
-                ss[c] = si[c] + d;
+                if (!DELTA) ss[c] = si[c] + d;
             }
         }
     } else {                                                    /* :132-135 */
@@ -337,7 +338,6 @@ __device__ __forceinline__ void stage_state(int j, const KRows &K, const double 
                 double acc = S.a[0] * K(S.r[0], c);
                 for (int i = 1; i < S.n; ++i) acc = acc + S.a[i] * K(S.r[i], c);
                 dl[c] = acc;
-                ss[c] = si[c] + acc;
             } else {
                 PtR acc = si[c];
 #if defined(PT_EXACT) && PT_SMUL_STAGE
@@ -408,13 +408,14 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
             const PtR d = dt * k4;
             dsf[c] = d;
             sf[c] = si[c] + d;
-            sr[c] = PtR(P.atol) + PtR(P.rtol) * pt_max(fabs(si[c]), fabs(sf[c]));
+            /* a NaN in either makes the norm NaN whichever the maximum is */
+            sr[c] = PtR(P.atol) + PtR(P.rtol) * pt_max_pos(fabs(si[c]), fabs(sf[c]));
         }
 #ifndef PT_EXACT
         if (P.noise != 0.0) {            /* PT_CTL_NOISE: sr += 2 |dt| nu per group, */
             /* |dt f|_max read off the step's increment dsf = dt k4 (registers) */
-            const double np_ = P.noise * pt_max(fabs(dsf[0]), pt_max(fabs(dsf[1]), fabs(dsf[2])));
-            const double nm_ = P.noise * pt_max(fabs(dsf[3]), pt_max(fabs(dsf[4]), fabs(dsf[5])));
+            const double np_ = P.noise * pt_max_pos(fabs(dsf[0]), pt_max_pos(fabs(dsf[1]), fabs(dsf[2])));
+            const double nm_ = P.noise * pt_max_pos(fabs(dsf[3]), pt_max_pos(fabs(dsf[4]), fabs(dsf[5])));
 #pragma unroll
             for (int c = 0; c < 6; ++c) sr[c] += (c < 3) ? np_ : nm_;
         }
@@ -449,11 +450,11 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
         const double deno = err5 + 1.0e-02 * err3;
 #ifdef PT_EXACT
         const double num = PtR(fabs(dt)) * err5;
-        return num / sqrt((deno <= 0.0) ? 6.0 : (double)(PtR(6.0) * deno));
+        return num / sqrt(pt_le(deno, 0.0) ? 6.0 : (double)(PtR(6.0) * deno));
 #else
         /* 1/sqrt(6) = 0.40824829046386307; the refined reciprocal square
          * root outside the subnormal range of its hardware approximation */
-        if (!(deno > 1.0e-300))
+        if (pt_le(deno, 1.0e-300))          /* NaN stays NaN below */
             return (deno <= 0.0) ? fabs(dt) * err5 * 0.40824829046386307
                                  : fabs(dt) * err5 / sqrt(6.0 * deno);
         return fabs(dt) * err5 * pt_rsqrt(6.0 * deno);
@@ -463,8 +464,8 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
 #ifndef PT_EXACT
         double nfl[2] = { 0.0, 0.0 };    /* PT_CTL_NOISE: (2 nu / atol) per group */
         if (P.noise != 0.0) {
-            nfl[0] = P.noise * pt_max(fabs(K(0, 0)), pt_max(fabs(K(0, 1)), fabs(K(0, 2))));
-            nfl[1] = P.noise * pt_max(fabs(K(0, 3)), pt_max(fabs(K(0, 4)), fabs(K(0, 5))));
+            nfl[0] = P.noise * pt_max_pos(fabs(K(0, 0)), pt_max_pos(fabs(K(0, 1)), fabs(K(0, 2))));
+            nfl[1] = P.noise * pt_max_pos(fabs(K(0, 3)), pt_max_pos(fabs(K(0, 4)), fabs(K(0, 5))));
         }
 #endif
 #pragma unroll
@@ -495,7 +496,7 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
             if (__double_as_longlong(sr) == 0) sr = 2.2250738585072014e-308;
 #endif
             const double q = fabs(PT_DIV(e, sr));
-            del = (c == 0) ? q : pt_nanmax(del, q);
+            del = (c == 0) ? q : pt_max_pos(del, q);    /* magnitudes: a NaN is the largest */
         }
         return PT_DIV(del, P.atol);
     }
@@ -701,10 +702,10 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
             /* ---- tail: finish the attempt that just ran ---- */
             if (active) {
                 q = finish_attempt<METHOD>(PT_Q, K, si, L.dt, pt, dl);
-                if (q != q) {
+                if (pt_isnan(q)) {
                     lane_close<METHOD>(PT_Q, K, L, si, PT_ST_NONFINITE, true);
                     active = false;
-                } else if (q <= 1.0) {
+                } else if (pt_le(q, 1.0)) {
                     mode = M_ACCEPT;
                     need = true;
                 } else {
@@ -884,7 +885,7 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                 }
             }
 #ifndef PT_EXACT
-            if (PT_Q.face && active) L.dt = pt_face_cap(PT_Q, si, L.dt);
+            if (PT_Q.face && active) L.dt = EV::face_cap(PT_Q, si, O, L.dt);
 #endif
             /* ---- start of the next attempt ---- */
             if (active) {

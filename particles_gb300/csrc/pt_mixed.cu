@@ -372,6 +372,12 @@ struct EvalMixed {
         for (int c = 1; c < 6; ++c) r = (Q.c == c) ? af[c] : r;
         return pt_f2d(r);
     }
+    /* the origin holds what the face cap needs of si */
+    static __device__ __forceinline__ double face_cap(const PtRun &P, const double *, const Origin &O,
+                                                      double h)
+    {
+        return pt_sm::pt_face_cap(P, O.off, O.u, h);
+    }
     static __device__ __forceinline__ double coop_face_cap(const PtRun &P, const pt_sm::Group &, double,
                                                            const Origin &O, double h)
     {
