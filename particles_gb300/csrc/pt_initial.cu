@@ -16,6 +16,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <math.h>
 #include <stdint.h>
 
@@ -64,18 +65,22 @@ __global__ void k_initial(const InitArgs A, double *__restrict__ state)
 #pragma unroll
         for (int c = 0; c < 3; ++c) s[c] = (A.hi[c] - A.lo[c]) * uniform01(A.seed, idx, c) + A.lo[c];
         if (A.kind == PT_INIT_MAXWELLIAN) {
+            /* The draws first, then the transform of the accepted one: a warp
+             * leaves the loop after about three draws, and with the logarithm,
+             * division and root inside it ran them that often for a few lanes
+             * each (1,000,003 particles 1.12 ms). */
             for (int c = 0; c < 3; ++c) {
-                double out = 0.0;
+                double u = 0.0, q = 0.0;
                 for (int d = 0; d < kMaxPolarDraws; ++d) {
-                    const double u = 2.0 * uniform01(A.seed, idx, 16 + 64 * c + 2 * d) - 1.0;
+                    u = 2.0 * uniform01(A.seed, idx, 16 + 64 * c + 2 * d) - 1.0;
                     const double v = 2.0 * uniform01(A.seed, idx, 17 + 64 * c + 2 * d) - 1.0;
-                    const double q = u * u + v * v;
-                    if (q > 0.0 && q <= 1.0) {
-                        out = u * sqrt(-2.0 * log(q) / q) * A.a;
-                        break;
-                    }
+                    q = u * u + v * v;
+                    /* 0 < q <= 1 on the bits (q >= +0) */
+                    const long long b = __double_as_longlong(q);
+                    if (b - 1 < 0x3ff0000000000000LL && b > 0) break;
+                    q = 0.0;
                 }
-                s[3 + c] = out;
+                s[3 + c] = (__double2hiint(q) != 0) ? u * sqrt(-2.0 * log(q) / q) * A.a : 0.0;
             }
         } else {
             const double mu = 2.0 * uniform01(A.seed, idx, 3) - 1.0;
@@ -102,71 +107,133 @@ __global__ void k_initial(const InitArgs A, double *__restrict__ state)
 
 /* ---- moments -------------------------------------------------------------- */
 
-constexpr int kMomBlocks = 256, kMomThreads = 256;
+constexpr int kMomBlocks = 304, kMomThreads = 256;
+/* doubles of one call's scratch: per block two (sum, compensation) pairs, the
+ * four moments, the arrival counter */
+constexpr int kMomScratch = 4 * kMomBlocks + 4 + 1;
 
-/* Neumaier accumulation of x into (s, c). */
+/* Neumaier accumulation of x into (s, c); magnitudes compared on their bits. */
 __device__ __forceinline__ void neu_add(double &s, double &c, double x)
 {
     const double t = s + x;
-    if (fabs(s) >= fabs(x)) c += (s - t) + x;
-    else c += (x - t) + s;
+    const bool ge = (__double_as_longlong(s) & 0x7fffffffffffffffLL) >=
+                    (__double_as_longlong(x) & 0x7fffffffffffffffLL);
+    const double a = ge ? s : x, b = ge ? x : s;
+    c += (a - t) + b;
     s = t;
 }
 
-/* Term of moment `mode` for value x given the moments found so far:
- * 0: x; 1: (x - mean)^2; 2: t^3, 3: t^4 with t = (x - mean) / sd (sd != 0). */
-__device__ __forceinline__ double mom_term(int mode, double x, const double *mom)
+/* One pass over the values.  PASS 0: sum of x; 1: of (x - mean)^2; 2: of t^3
+ * and t^4 with t = (x - mean) / sd (x - mean where sd is 0).
+ *
+ * What bounds a pass is the FP64 pipe: 4 operations per Neumaier step, up to
+ * 15 per value in pass 2 (the quotient through one reciprocal, pt_qdiv).  Fixed
+ * partition: block b sums a contiguous chunk, thread j every blockDim-th
+ * element of it, and a block combines its threads in a fixed tree; the block
+ * that arrives last combines the blocks in the same way and finishes the
+ * moments, so a moment takes one launch and its bits do not depend on the
+ * order of arrival. */
+template <int PASS>
+__global__ void __launch_bounds__(kMomThreads) k_moments(int64_t n, const double *__restrict__ x,
+                                                         int64_t stride, double *scratch)
 {
-    if (mode == 0) return x;
-    double t = x - mom[0];
-    if (mode == 1) return t * t;
-    if (mom[1] != 0.0) t = t / mom[1];
-    return (mode == 2) ? t * t * t : (t * t) * (t * t);
-}
-
-/* Fixed partition: block b sums a contiguous chunk, thread j every
- * blockDim-th element of it; the block combines its threads in a fixed tree.
- * part[2b], part[2b+1] = the block's (sum, compensation). */
-__global__ void __launch_bounds__(kMomThreads) k_mom_partial(int mode, int64_t n,
-                                                             const double *__restrict__ x,
-                                                             int64_t stride, const double *mom,
-                                                             double *part)
-{
-    __shared__ double ss[kMomThreads], sc[kMomThreads];
-    const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t b0 = blockIdx.x * chunk;
-    const int64_t b1 = (b0 + chunk < n) ? b0 + chunk : n;
-    double s = 0.0, c = 0.0;
-    for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) neu_add(s, c, mom_term(mode, x[i * stride], mom));
-    ss[threadIdx.x] = s;
-    sc[threadIdx.x] = c;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) {
-            double a = ss[threadIdx.x], ac = sc[threadIdx.x] + sc[threadIdx.x + h];
-            neu_add(a, ac, ss[threadIdx.x + h]);
-            ss[threadIdx.x] = a;
-            sc[threadIdx.x] = ac;
+    __shared__ double ss[2][kMomThreads], sc[2][kMomThreads];
+    __shared__ bool last;
+    double *const part = scratch, *const mom = scratch + 4 * kMomBlocks;
+    unsigned long long *const arrived = reinterpret_cast<unsigned long long *>(mom + 4);
+    constexpr int NS = PASS == 2 ? 2 : 1;
+    double s[2] = { 0.0, 0.0 }, c[2] = { 0.0, 0.0 };
+    const int tid = threadIdx.x;
+    {
+        const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
+        const int64_t b0 = blockIdx.x * chunk;
+        const int64_t b1 = (b0 + chunk < n) ? b0 + chunk : n;
+        const double mean = PASS > 0 ? mom[0] : 0.0;
+        const double sd = (PASS == 2 && mom[1] != 0.0) ? mom[1] : 1.0, ysd = 1.0 / sd;
+#pragma unroll 4
+        for (int64_t i = b0 + tid; i < b1; i += kMomThreads) {
+            const double v = x[i * stride];
+            if (PASS == 0) {
+                neu_add(s[0], c[0], v);
+            } else {
+                double t = v - mean;
+                if (PASS == 1) {
+                    neu_add(s[0], c[0], t * t);
+                } else {
+                    t = pt_qdiv(t, sd, ysd);
+                    const double t2 = t * t;
+                    neu_add(s[0], c[0], t2 * t);
+                    neu_add(s[1], c[1], t2 * t2);
+                }
+            }
         }
-        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = ss[0];
-        part[2 * blockIdx.x + 1] = sc[0];
+    auto tree = [&]() {
+#pragma unroll
+        for (int k = 0; k < NS; ++k) { ss[k][tid] = s[k]; sc[k][tid] = c[k]; }
+        __syncthreads();
+        for (int h = kMomThreads / 2; h > 0; h >>= 1) {
+            if (tid < h * NS) {
+                const int k = NS == 2 ? tid / h : 0, i = NS == 2 ? tid % h : tid;
+                double a = ss[k][i], ac = sc[k][i] + sc[k][i + h];
+                neu_add(a, ac, ss[k][i + h]);
+                ss[k][i] = a;
+                sc[k][i] = ac;
+            }
+            __syncthreads();
+        }
+    };
+    tree();
+    if (tid == 0) {
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            part[4 * blockIdx.x + 2 * k] = ss[k][0];
+            part[4 * blockIdx.x + 2 * k + 1] = sc[k][0];
+        }
+        __threadfence();
+        last = atomicAdd(arrived, 1ULL) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    /* the last block: thread j takes blocks j, j + 256, then the same tree */
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        s[k] = c[k] = 0.0;
+        for (int b = tid; b < (int)gridDim.x; b += kMomThreads) {
+            c[k] += __ldcg(part + 4 * b + 2 * k + 1);
+            neu_add(s[k], c[k], __ldcg(part + 4 * b + 2 * k));
+        }
+    }
+    __syncthreads();
+    tree();
+    if (tid == 0) {
+        const double m0 = (ss[0][0] + sc[0][0]) / (double)n;
+        if (PASS == 2) {
+            mom[2] = m0;
+            mom[3] = (ss[1][0] + sc[1][0]) / (double)n - 3.0;
+        } else {
+            mom[PASS] = PASS == 1 ? sqrt(m0) : m0;
+        }
+        *arrived = 0ULL;
     }
 }
 
-/* One thread: the blocks' partial sums in block order, then moment `mode`. */
-__global__ void k_mom_finish(int mode, int64_t n, int nb, const double *part, double *mom)
+/* Scratch of pt_moments calls: the call returns after its stream is done, so
+ * a slot serves one call at a time; more calls at once than slots allocate. */
+constexpr int kMomSlots = 8;
+__device__ double g_mom_scratch[kMomSlots][kMomScratch];
+std::atomic<uint32_t> g_mom_taken{ 0 };
+
+int mom_take()
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0, c = 0.0;
-    for (int b = 0; b < nb; ++b) {
-        c += part[2 * b + 1];
-        neu_add(s, c, part[2 * b]);
+    uint32_t t = g_mom_taken.load(std::memory_order_relaxed);
+    for (;;) {
+        int k = 0;
+        while (k < kMomSlots && ((t >> k) & 1u)) ++k;
+        if (k == kMomSlots) return -1;
+        if (g_mom_taken.compare_exchange_weak(t, t | (1u << k), std::memory_order_acquire)) return k;
     }
-    const double mean = (s + c) / (double)n;
-    mom[mode] = (mode == 1) ? sqrt(mean) : (mode == 3) ? mean - 3.0 : mean;
 }
 
 }  // namespace
@@ -212,18 +279,29 @@ extern "C" int pt_moments(int64_t n, const double *d_x, int64_t stride, double o
 {
     if (n < 1 || !d_x || stride < 1 || !out) return set_err(PT_ERR_ARG, "pt_moments: bad arguments%s", "");
     cudaStream_t s = (cudaStream_t)stream;
-    double *buf = nullptr;                     /* partials, then the 4 moments */
-    cudaError_t e = cudaMalloc(&buf, (2 * kMomBlocks + 4) * sizeof(double));
-    if (e != cudaSuccess) return cuda_err(e, "pt_moments");
-    double *mom = buf + 2 * kMomBlocks;
-    e = cudaMemsetAsync(mom, 0, 4 * sizeof(double), s);
-    for (int mode = 0; mode < 4 && e == cudaSuccess; ++mode) {
-        k_mom_partial<<<kMomBlocks, kMomThreads, 0, s>>>(mode, n, d_x, stride, mom, buf);
-        k_mom_finish<<<1, 32, 0, s>>>(mode, n, kMomBlocks, buf, mom);
+    const int slot = mom_take();
+    double *buf = nullptr;
+    cudaError_t e;
+    if (slot >= 0) {
+        e = cudaGetSymbolAddress(reinterpret_cast<void **>(&buf), g_mom_scratch);
+        buf += (size_t)slot * kMomScratch;
+    } else {
+        e = cudaMalloc(&buf, kMomScratch * sizeof(double));
+    }
+    double *mom = buf + 4 * kMomBlocks;
+    if (e == cudaSuccess) e = cudaMemsetAsync(mom, 0, 5 * sizeof(double), s);
+    if (e == cudaSuccess) {
+        const int64_t need = (n + kMomThreads - 1) / kMomThreads;
+        const int grid = (int)(need < kMomBlocks ? need : kMomBlocks);
+        k_moments<0><<<grid, kMomThreads, 0, s>>>(n, d_x, stride, buf);
+        k_moments<1><<<grid, kMomThreads, 0, s>>>(n, d_x, stride, buf);
+        k_moments<2><<<grid, kMomThreads, 0, s>>>(n, d_x, stride, buf);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, mom, 4 * sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(buf);
+    const cudaError_t w = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = w;
+    if (slot >= 0) g_mom_taken.fetch_and(~(1u << slot), std::memory_order_release);
+    else cudaFree(buf);
     return e == cudaSuccess ? PT_OK : cuda_err(e, "pt_moments");
 }

@@ -87,3 +87,25 @@ def test_moments_edge_cases(cuda):
     assert np.array_equal(initial.moments_on_device(one), initial.moments(np.array([2.5])))
     const = cuda.full((1000,), 1.25, dtype=cuda.float64, device="cuda")
     assert np.array_equal(initial.moments_on_device(const), np.array([1.25, 0.0, 0.0, -3.0]))
+
+
+@pytest.mark.parametrize("n", [2, 255, 257, 304 * 256, 304 * 256 + 1, 300007])
+def test_moments_over_the_partition(cuda, n):
+    """Sizes around the blocks' partition, from twelve threads at once (more
+    than the calls that share the scratch slots), against long double sums.
+    Compensated sums of n terms, each term within a few roundings: 16 eps of
+    the sum of magnitudes."""
+    from concurrent.futures import ThreadPoolExecutor
+    h = np.random.default_rng(n).normal(3.0, 0.7, n)
+    x = cuda.tensor(h, device="cuda")
+    cuda.cuda.synchronize()
+    with ThreadPoolExecutor(12) as ex:
+        got = list(ex.map(lambda _: initial.moments_on_device(x), range(24)))
+    assert all(np.array_equal(g, got[0]) for g in got)
+    w = h.astype(np.longdouble)
+    mean = w.mean()
+    sd = np.sqrt(((w - mean) ** 2).mean())
+    t = (w - mean) / sd
+    ref = np.array([mean, sd, (t ** 3).mean(), (t ** 4).mean() - 3], np.float64)
+    scale = np.array([np.abs(w).mean(), sd, (np.abs(t) ** 3).mean(), (t ** 4).mean()], np.float64)
+    assert np.all(np.abs(got[0] - ref) <= 16 * 2.0 ** -52 * scale), (got[0] - ref) / scale
