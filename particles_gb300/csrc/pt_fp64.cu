@@ -296,16 +296,14 @@ struct CoopF64 : EvalF64<NC> {
         const int32_t r = (l + 1 == dm) ? 0 : l + 1;
         const double xd = xn - fl, xu = 1.0 - xd;
 #endif
-        /* lane q's corner: x from bit 2, y from bit 1, z from bit 0 of q; an
-         * index fits 16 bits (dm <= 2^16) */
-        const uint32_t lr = (uint32_t)l | ((uint32_t)r << 16);
+        /* lane q's corner: x from bit 2, y from bit 1, z from bit 0 of q */
         int32_t ix[3];
         PtR w;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const bool right = (G.gl >> (2 - i)) & 1;
-            const uint32_t v = G.get(lr, i);
-            ix[i] = (int32_t)(right ? v >> 16 : v & 0xffffu);
+            const int32_t il = G.get(l, i), ir = G.get(r, i);
+            ix[i] = right ? ir : il;
             const double d = G.get(xd, i), u = G.get(xu, i);
             const double f = right ? d : u;
             w = (i == 0) ? PtR(f) : w * f;

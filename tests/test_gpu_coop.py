@@ -99,3 +99,34 @@ def test_ensemble_of_few_and_many(cuda, oracle_lib):
             so, co, _ = oracle.integrate("dop853", p["params"], p["time"], *p["fields"], p["state"].copy())
             assert np.array_equal(m["cnt"].cpu().numpy(), co)
             assert np.array_equal(m["state"].cpu().numpy().view(np.int64), so.view(np.int64))
+
+
+def test_noalloc_grid_longer_than_16_bits(cuda, oracle_lib):
+    """The no-allocation entry point takes axes of up to 64^3 nodes: node
+    indices beyond 2^16 in the eight-lane gather."""
+    torch = cuda
+    import ctypes as C
+    import oracle
+    from particles_gb300 import _native as N
+    from particles_gb300 import initial, params
+    dm = (100003, 1, 2)
+    rng = np.random.default_rng(7)
+    uu = 0.01 * rng.normal(size=(3, 2, 1, dm[0]))
+    bb = 0.1 * rng.normal(size=uu.shape)
+    bb[0] += 1.0
+    tmax = 1e-3 * 2 * np.pi / 200.0
+    prm = params.pack_params(qom=200.0, vunit=0.05, tmax=tmax, dtmax=tmax, atol=1e-6, rtol=1e-6)
+    tg = params.time_grid(2, tmax)
+    st = np.zeros((40, tg.size, 8))
+    st[:, 0, :6] = initial.isotropic_state(40, 9, speed=0.5)
+    so, co, _ = oracle.integrate("rk5", prm, tg, uu, bb, st.copy())
+    t = lambda a: torch.tensor(a, device="cuda")
+    p = lambda a: C.c_void_p(a.data_ptr())
+    d = dict(t=t(tg), u=t(uu), b=t(bb), s=t(st), c=torch.zeros((40, 3), dtype=torch.int64, device="cuda"))
+    L = N.load()
+    N.check(L.pt_integrate_device_noalloc(1, 40, tg.size, np.array(dm, np.int32).ctypes.data_as(C.c_void_p),
+                                          prm.ctypes.data_as(C.c_void_p), p(d["t"]), p(d["u"]), p(d["b"]),
+                                          p(d["s"]), p(d["c"]), None, None), "noalloc")
+    assert L.pt_integrate_device_noalloc_check(None) == 0
+    assert np.array_equal(d["c"].cpu().numpy(), co)
+    assert np.array_equal(d["s"].cpu().numpy().view(np.int64), so.view(np.int64))
