@@ -61,9 +61,15 @@ struct KOwn {
 /* Shared memory per block: k rows, then the gather's transpose area (per
  * group NV rows of 8 products, rows padded to 9). */
 template <int METHOD, class EV>
-__host__ __device__ constexpr int coop_smem_bytes(int block)
+__host__ __device__ constexpr int coop_rows_bytes(int block)
 {
     return Traits<METHOD>::ROWS * 8 * block + EV::kCoopRows * 9 * 8 * (block / kGroup);
+}
+/* ... and, with a learned controller, its weight blob. */
+template <int METHOD, class EV>
+__host__ __device__ constexpr int coop_smem_bytes(int block, bool learn)
+{
+    return coop_rows_bytes<METHOD, EV>(block) + (learn ? PT_MLP_BLOB_BYTES : 0);
 }
 
 template <int METHOD>
@@ -317,7 +323,7 @@ __device__ __forceinline__ double coop_finish(const PtRun &P, const Group &G, co
 
 /* from_queue: particles come from the work queue; then, and otherwise only,
  * from the hand-over list of the launch before (complete: that launch is over). */
-template <int METHOD, class EV, bool ENS = false>
+template <int METHOD, class EV, bool LEARN, bool ENS = false>
 __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue)
 {
     using T = Traits<METHOD>;
@@ -327,6 +333,8 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
     double *const tr = pt_ksm + T::ROWS * blockDim.x + (threadIdx.x / kGroup) * (EV::kCoopRows * 9);
     int mi = 0;
 #define PT_Q (MB.q(mi))
+    unsigned char *const blob = reinterpret_cast<unsigned char *>(pt_ksm) + coop_rows_bytes<METHOD, EV>(blockDim.x);
+    if (LEARN) (void)pt_mlp_load(PT_Q.mlp, blob);
     uint64_t t_start = pt_globaltimer();
     const PtHand H = MB.q(0).hand;
     const unsigned long long handed = H.ctl ? H.ctl[0] : 0ULL;
@@ -417,6 +425,7 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
             }
         } else {
             const double dt = L.dt;
+            const bool was_rejected = L.rejected;
             double fpow = 0.0;
             if (mode == M_ACCEPT || mode == M_REJECT) {
                 const double y = (METHOD == PT_METHOD_DOP853) ? PT_Q.expo
@@ -472,6 +481,38 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
                 next_time(PT_Q, L);
             }
             if (active && (mode == M_ACCEPT || mode == M_READY)) EV::coop_begin(PT_Q, G, si, O);
+            if constexpr (LEARN) {
+                /* as in run_machine: the group's lanes form the features alike,
+                 * its first lane is the row of the network's input */
+                const bool want = (mode == M_ACCEPT) && active;
+                float feat[PT_REC_NFEAT] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
+                if (want) {
+                    double s6[6];
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) s6[c] = G.get(si, c);
+                    int32_t fl_[3], fr_[3];
+                    float fx_[3];
+                    EV::feature_cell(PT_Q, s6, O, fl_, fr_, fx_);
+                    const auto ld_ = EV::feature_loader(PT_Q, fl_, fr_);
+                    pt_field_features(PT_Q, ld_, s6, fx_, feat);
+                    const float om = PT_Q.qomf * __expf(feat[0] - feat[2]);
+                    const float dtf = pt_d2f(dt);
+                    feat[5] = __logf(om * dtf + 1e-30f);
+                    feat[6] = __logf(pt_d2f(q) + 1e-30f);
+                    feat[7] = __logf(dtf);
+                    feat[8] = __logf(fminf(pt_face_time(PT_Q, s6, fx_) / dtf, 1.0e6f) + 1e-30f);
+                }
+                if (__any_sync(0xffffffffu, want)) {
+                    const float y = G.get(pt_mlp_warp(pt_mlp_view(blob), feat, want && G.gl == 0), 0);
+                    if (want) {
+                        const double lo = PT_Q.fcmn * dt;
+                        const double hi = (METHOD == PT_METHOD_DOP853 && was_rejected) ? dt : PT_Q.fcmx * dt;
+                        const double h = pt_f2d(__expf(y));
+                        L.dt = pt_min(pt_max(h, lo), hi);
+                        L.dt = pt_min(L.dt, PT_Q.dtm);
+                    }
+                }
+            }
 #ifndef PT_EXACT
             /* a handed-over step is capped already */
             if (PT_Q.face && active && !handed_over) L.dt = EV::coop_face_cap(PT_Q, G, si, O, L.dt);
@@ -519,14 +560,14 @@ inline int coop_sms()
  * the GPU).  Runs of under four groups per scheduler take one-warp blocks,
  * which spread over all SMs. */
 template <int METHOD, class EV, class KERN, class... Args>
-cudaError_t launch_coop(KERN kern, int64_t n, cudaStream_t s, Args... args)
+cudaError_t launch_coop(KERN kern, int64_t n, bool learn, cudaStream_t s, Args... args)
 {
     const int sms = coop_sms();
     const int block = (n >= 0 && n < 16 * (int64_t)sms) ? 32 : 128;
     const int64_t full = (int64_t)sms * 3;
     int64_t grid = n < 0 ? full : (n * kGroup + block - 1) / block;
     if (block == 128 && grid > full) grid = full;
-    kern<<<(int)(grid < 1 ? 1 : grid), block, coop_smem_bytes<METHOD, EV>(block), s>>>(args...);
+    kern<<<(int)(grid < 1 ? 1 : grid), block, coop_smem_bytes<METHOD, EV>(block, learn), s>>>(args...);
     return cudaGetLastError();
 }
 

@@ -252,7 +252,7 @@ struct EvalF64 {
 template <int NC>
 struct CoopF64 : EvalF64<NC> {
     static constexpr int NV = (NC == 10) ? 9 : 6;
-    struct CoopOrigin {};
+    using CoopOrigin = typename EvalF64<NC>::Origin;
 #ifdef PT_EXACT
     static constexpr int kCoopRows = NV;           /* products */
 #else
@@ -403,10 +403,10 @@ struct CoopF64 : EvalF64<NC> {
     }
 };
 
-template <int METHOD, int NC>
+template <int METHOD, int NC, bool LEARN>
 __global__ void __launch_bounds__(128, 3) k_coop(const PtRun P, bool from_queue)
 {
-    pt_sm::run_coop<METHOD, CoopF64<NC>>(pt_sm::Members<false>{ P }, from_queue);
+    pt_sm::run_coop<METHOD, CoopF64<NC>, LEARN>(pt_sm::Members<false>{ P }, from_queue);
 }
 
 template <int METHOD, int NC>
@@ -417,14 +417,14 @@ __global__ void __launch_bounds__(128, 3) k_ensemble_coop(const PtRun *__restric
     __shared__ int64_t sN[PT_ENS_MAX];
     pt_sm::ens_load(tab, nmem, sP, sN);
     const pt_sm::Members<true> MB{ sP, sN, nmem };
-    pt_sm::run_coop<METHOD, CoopF64<NC>, true>(MB, MB.total() <= few);
+    pt_sm::run_coop<METHOD, CoopF64<NC>, false, true>(MB, MB.total() <= few);
 }
 
 template <int METHOD, int NC, bool LEARN, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
 k_integrate(const PtRun P)
 {
-    pt_sm::run_machine<METHOD, EvalF64<NC>, LEARN, false, !LEARN>(pt_sm::Members<false>{ P });
+    pt_sm::run_machine<METHOD, EvalF64<NC>, LEARN, false, true>(pt_sm::Members<false>{ P });
 }
 
 /* Several runs (members: snapshots, tolerances, particle sets) in one
@@ -512,7 +512,7 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
     /* how many particles are left is known on the device only: both kernels
      * are launched, and the one that is not to take the queue finds nothing */
     if (e == cudaSuccess && ntot > 0)
-        e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_ensemble_coop<METHOD, NC>, -1, s, tab, nmem,
+        e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_ensemble_coop<METHOD, NC>, -1, false, s, tab, nmem,
                                                     (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
     return e;
 }
@@ -531,11 +531,13 @@ template <int METHOD, int NC>
 cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
-    if (P.mlp || P.rec) return launch_v<METHOD, NC, true>(P, s);
+    if (P.rec) return launch_v<METHOD, NC, true>(P, s);
     const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
-    cudaError_t e = few ? cudaSuccess : launch_v<METHOD, NC, false>(P, s);
-    if (e == cudaSuccess && (few || P.hand.ctl))
-        e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC>, few ? P.np : -1, s, P, few);
+    cudaError_t e = few ? cudaSuccess : P.mlp ? launch_v<METHOD, NC, true>(P, s) : launch_v<METHOD, NC, false>(P, s);
+    if (e == cudaSuccess && (few || P.hand.ctl)) {
+        if (P.mlp) e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC, true>, few ? P.np : -1, true, s, P, few);
+        else e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC, false>, few ? P.np : -1, false, s, P, few);
+    }
     return e;
 }
 

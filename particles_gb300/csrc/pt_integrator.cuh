@@ -907,7 +907,7 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
             }
             if (HAND && __popc(act) <= PT_HAND_LANES && __any_sync(0xffffffffu, drained)) {
                 const PtHand H = MB.q(0).hand;
-                if (H.ctl) {
+                if (H.ctl && !(LEARN && MB.q(0).rec)) {   /* recording keeps its pending records */
                     const int lane = threadIdx.x & 31;
                     unsigned long long at = 0;
                     if (lane == 0) at = atomicAdd(H.ctl, (unsigned long long)__popc(act));

@@ -389,13 +389,13 @@ template <int METHOD, class EV, bool LEARN, int MINB>
 __global__ void __launch_bounds__(PT_BLOCK_MAX) __maxnreg__(PT_REGS_OF_MINB(MINB))
 k_integrate_mixed(const PtRun P)
 {
-    pt_sm::run_machine<METHOD, EV, LEARN, false, !LEARN>(pt_sm::Members<false>{ P });
+    pt_sm::run_machine<METHOD, EV, LEARN, false, true>(pt_sm::Members<false>{ P });
 }
 
-template <int METHOD, class EV>
+template <int METHOD, class EV, bool LEARN>
 __global__ void __launch_bounds__(128, 3) k_coop_mixed(const PtRun P, bool from_queue)
 {
-    pt_sm::run_coop<METHOD, EV>(pt_sm::Members<false>{ P }, from_queue);
+    pt_sm::run_coop<METHOD, EV, LEARN>(pt_sm::Members<false>{ P }, from_queue);
 }
 
 template <int METHOD, class EV>
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(128, 3) k_ensemble_coop_mixed(const PtRun *__r
     __shared__ int64_t sN[PT_ENS_MAX];
     pt_sm::ens_load(tab, nmem, sP, sN);
     const pt_sm::Members<true> MB{ sP, sN, nmem };
-    pt_sm::run_coop<METHOD, EV, true>(MB, MB.total() <= few);
+    pt_sm::run_coop<METHOD, EV, false, true>(MB, MB.total() <= few);
 }
 
 /* Several runs (members: snapshots, tolerances, particle sets) in one
@@ -479,7 +479,7 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
     /* how many particles are left is known on the device only: both kernels
      * are launched, and the one that is not to take the queue finds nothing */
     if (e == cudaSuccess && ntot > 0)
-        e = pt_sm::launch_coop<METHOD, EV>(k_ensemble_coop_mixed<METHOD, EV>, -1, s, tab, nmem,
+        e = pt_sm::launch_coop<METHOD, EV>(k_ensemble_coop_mixed<METHOD, EV>, -1, false, s, tab, nmem,
                                            (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
     return e;
 }
@@ -499,11 +499,14 @@ template <int METHOD, class EV, bool LEARNABLE>
 cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
-    if (LEARNABLE && (P.mlp || P.rec)) return launch_v<METHOD, EV, LEARNABLE>(P, s);
+    if (LEARNABLE && P.rec) return launch_v<METHOD, EV, LEARNABLE>(P, s);
+    const bool learn = LEARNABLE && P.mlp;
     const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
-    cudaError_t e = few ? cudaSuccess : launch_v<METHOD, EV, false>(P, s);
-    if (e == cudaSuccess && (few || P.hand.ctl))
-        e = pt_sm::launch_coop<METHOD, EV>(k_coop_mixed<METHOD, EV>, few ? P.np : -1, s, P, few);
+    cudaError_t e = few ? cudaSuccess : learn ? launch_v<METHOD, EV, LEARNABLE>(P, s) : launch_v<METHOD, EV, false>(P, s);
+    if (e == cudaSuccess && (few || P.hand.ctl)) {
+        if (learn) e = pt_sm::launch_coop<METHOD, EV>(k_coop_mixed<METHOD, EV, LEARNABLE>, few ? P.np : -1, true, s, P, few);
+        else e = pt_sm::launch_coop<METHOD, EV>(k_coop_mixed<METHOD, EV, false>, few ? P.np : -1, false, s, P, few);
+    }
     return e;
 }
 

@@ -48,15 +48,21 @@ def test_exact_bitwise_at_every_size(cuda, oracle_lib, method, with_j, near, siz
 @pytest.mark.parametrize("method,tol", [("rk5", 1e-8), ("dop853", 1e-8)])
 @pytest.mark.parametrize("prec,kw", [("fp64_fma", {}), ("fp64_fma", dict(face_steps=True)), ("fp32", {}),
                                      ("fp32", dict(face_steps=True, noise_floor=True)),
-                                     ("bf16", dict(noise_floor=True))])
+                                     ("bf16", dict(noise_floor=True)),
+                                     ("fp64", dict(learned=True)), ("fp64_fma", dict(learned=True)),
+                                     ("fp32", dict(learned=True, face_steps=True))])
 @pytest.mark.parametrize("with_j", [False, True])
 def test_both_machines_give_the_same_bits(cuda, method, tol, prec, kw, with_j):
     """A particle's result does not depend on how many others run with it: a
     few of them alone (eight lanes throughout) against the same ones in a run
     that starts on one lane each and hands over."""
     torch = cuda
-    from particles_gb300 import Fields
+    from particles_gb300 import Fields, learned
     few = 333
+    kw = dict(kw)
+    if kw.pop("learned", False):
+        norm = np.concatenate([np.zeros(9), np.full(9, 3.0), [-8.0, 1.0]]).astype(np.float32)
+        kw["model"] = learned.Model(learned.init_params(5), norm, safety=0.9)
     npart = 3 * PER_SM * torch.cuda.get_device_properties(0).multi_processor_count + 17
     prob = small_problem(method, n=20, npart=npart, periods=0.1, seed=72, with_j=with_j, nsteps=7,
                          gamma_range=(1.001, 50.0), tol=tol)
