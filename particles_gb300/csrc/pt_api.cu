@@ -100,6 +100,7 @@ void unpack_params(const double *p, const RunShape &g, PtRun &R)
     }
     R.unit_map = unit ? 1 : 0;
     R.inv_vun = 1.0 / R.vun;
+    R.inv_atol = 1.0 / R.atol;
     R.ivunf = (float)R.inv_vun;
     R.qomf = (float)R.qom;
 }

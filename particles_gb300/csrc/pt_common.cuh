@@ -52,6 +52,7 @@ struct PtRun {
     double gsx[3], gox[3];  /* node coordinate = x * gsx + gox = (x - xl) / xs * dm */
     double inv_vun;         /* 1 / vun, correctly rounded */
     double inv_xs[3];       /* 1 / xs, correctly rounded */
+    double inv_atol;        /* 1 / atol, correctly rounded */
     float gsxf[3];          /* gsx rounded to FP32 (mixed precision) */
     float ivunf, qomf, etaf;
     int32_t dm[3];
@@ -209,6 +210,38 @@ __device__ __forceinline__ int32_t pt_node_index(double q, int32_t d)
     const uint32_t m = (hi & 0xfffffu) | 0x100000u;
     const int32_t v = (int32_t)(e < 20u ? m >> (20u - e) : __funnelshift_l(lo, m, e - 20u));
     return v < d ? v : 0;
+}
+
+/* The exact build's cell of one axis (interpolations.F90:140-149): left and
+ * right node of the scaled position x on d nodes, and the offset xd from the
+ * left one.  The reference forms the right node from x + 1/d the way it forms
+ * the left one from x; that is the left one's neighbour unless xd comes within
+ * rounding of 0 or 1.  With |x| < 2^10 and d <= 2^18 the two ways' coordinates
+ * differ from one node by at most d 2^-43 + d 2^-51 < 2^-24 (1/d rounded, x + 1/d
+ * rounded, then the fraction and the product), so for xd in [2^-20, 1 - 2^-20) the
+ * neighbour it is, at three FP64 operations, two floors and an index less per
+ * axis; else the reference's own steps decide.  mask = d - 1 for a power of two
+ * (else 0): the product by d is then an addition to the exponent. */
+__device__ __forceinline__ void pt_axis_exact(double x, int32_t d, int32_t mask, double dmr,
+                                              double inv_d, int32_t &l, int32_t &r, double &xd)
+{
+    auto times_d = [&](double fr) {
+        const uint32_t hi = (uint32_t)__double2hiint(fr);
+        if (mask && hi - 0x00100000u <= 0x3ff00000u - 0x00100000u)   /* normal, at most 1 */
+            return __hiloint2double((int)(hi + ((uint32_t)__popc(mask) << 20)), __double2loint(fr));
+        return pt_fmul(dmr, fr);
+    };
+    const double xp = times_d(pt_fsub(x, pt_floor(x)));
+    const double pl = pt_floor(xp);
+    l = pt_node_index(pl, d);
+    xd = pt_fsub(xp, pl);
+    const uint32_t hx = (uint32_t)__double2hiint(x) & 0x7fffffffu, hd = (uint32_t)__double2hiint(xd);
+    if (hx < 0x40900000u && hd - 0x3eb00000u < 0x3feffffeu - 0x3eb00000u) {
+        r = (l + 1 == d) ? 0 : l + 1;
+    } else {
+        const double xr = pt_fadd(x, inv_d);
+        r = pt_node_index(pt_floor(times_d(pt_fsub(xr, pt_floor(xr)))), d);
+    }
 }
 
 /* a / b correctly rounded from y = RN(1/b) (Markstein's quotient correction,

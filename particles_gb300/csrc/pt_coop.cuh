@@ -317,7 +317,11 @@ __device__ __forceinline__ double coop_finish(const PtRun &P, const Group &G, co
             const unsigned long long v = G.get(q, i);
             del = v > del ? v : del;
         }
+#ifdef PT_EXACT
+        return pt_qdiv(__longlong_as_double((long long)del), P.atol, P.inv_atol);
+#else
         return PT_DIV(__longlong_as_double((long long)del), P.atol);
+#endif
     }
 }
 

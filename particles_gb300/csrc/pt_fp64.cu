@@ -105,14 +105,10 @@ struct EvalF64 {
 #ifdef PT_EXACT
 #pragma unroll
         for (int i = 0; i < 3; ++i) {                            /* :140-149 */
-            const PtR x = P.unit_map ? s[i] : pt_qdiv(pt_fsub(s[i], P.xl[i]), P.xs[i], P.inv_xs[i]);
-            const PtR xr = x + P.inv_dm[i];
-            PtR xp = P.dmr[i] * (xr - pt_floor(xr));
-            r[i] = pt_node_index(pt_floor(xp), P.dm[i]);
-            xp = P.dmr[i] * (x - pt_floor(x));
-            const PtR pl = pt_floor(xp);
-            l[i] = pt_node_index(pl, P.dm[i]);
-            xd[i] = xp - pl;
+            const double x = P.unit_map ? s[i] : pt_qdiv(pt_fsub(s[i], P.xl[i]), P.xs[i], P.inv_xs[i]);
+            double o;
+            pt_axis_exact(x, P.dm[i], P.dm_mask[i], P.dmr[i], P.inv_dm[i], l[i], r[i], o);
+            xd[i] = o;
             xu[i] = 1.0 - xd[i];
         }
 #else
@@ -273,14 +269,10 @@ struct CoopF64 : EvalF64<NC> {
     {
         /* the cell and offset of the lane's axis (lanes 0-2; the others' values are unused) */
 #ifdef PT_EXACT
-        const PtR x = P.unit_map ? s : pt_qdiv(pt_fsub(s, P.xl[G.ax]), P.xs[G.ax], P.inv_xs[G.ax]);
-        const PtR xr = x + P.inv_dm[G.ax];
-        PtR xp = P.dmr[G.ax] * (xr - pt_floor(xr));
-        const int32_t r = pt_node_index(pt_floor(xp), P.dm[G.ax]);
-        xp = P.dmr[G.ax] * (x - pt_floor(x));
-        const PtR pl = pt_floor(xp);
-        const int32_t l = pt_node_index(pl, P.dm[G.ax]);
-        const double xd = xp - pl;
+        const double x = P.unit_map ? s : pt_qdiv(pt_fsub(s, P.xl[G.ax]), P.xs[G.ax], P.inv_xs[G.ax]);
+        int32_t l, r;
+        double xd;
+        pt_axis_exact(x, P.dm[G.ax], P.dm_mask[G.ax], P.dmr[G.ax], P.inv_dm[G.ax], l, r, xd);
         const double xu = PtR(1.0) - xd;
 #else
         const double xn = fma(s, P.gsx[G.ax], P.gox[G.ax]);

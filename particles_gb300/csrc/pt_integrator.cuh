@@ -498,7 +498,11 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
             const double q = fabs(PT_DIV(e, sr));
             del = (c == 0) ? q : pt_max_pos(del, q);    /* magnitudes: a NaN is the largest */
         }
+#ifdef PT_EXACT
+        return pt_qdiv(del, P.atol, P.inv_atol);
+#else
         return PT_DIV(del, P.atol);
+#endif
     }
 }
 
