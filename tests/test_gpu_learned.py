@@ -141,3 +141,32 @@ def test_learned_controller_in_the_integrator(cuda, oracle_lib):
     assert att["learned"] < att["classical"]
     for mdl in models.values():
         mdl.close()
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (15, 0), (17, 1), (127, 0), (128, 0), (129, 3), (304 * 128 + 5, 0)])
+def test_training_gradient_over_the_tiles(cuda, n, shift):
+    """Row counts around the warps' 16 rows, the blocks' 128 and the grid, and
+    gradient buffers off the 16-byte boundary.  Targets away from the outputs:
+    then a row's gradient carries the FP16 operands' rounding (2^-11 per layer)
+    and no cancellation, and stays within the bounds of the test above."""
+    torch = cuda
+    from oracle import mlp
+    from particles_gb300 import _native as N
+    L = N.load()
+    rng = np.random.default_rng(n)
+    p = (mlp.init_params(2) + rng.normal(0, 0.05, mlp.NPARAM)).astype(np.float32)
+    X = rng.normal(size=(n, 9)).astype(np.float32)
+    T = (4.0 + rng.normal(size=n)).astype(np.float32)
+    dp, dX, dT = (torch.tensor(a, device="cuda") for a in (p, X, T))
+    buf = torch.full((mlp.NPARAM + 8,), 7.0, device="cuda")      # stale values, and guards
+    g = buf[shift:shift + mlp.NPARAM]
+    loss = torch.full((1,), 7.0, device="cuda")
+    vp = lambda t: C.c_void_p(t.data_ptr())
+    N.check(L.pt_mlp_loss_grad(vp(dp), vp(dX), vp(dT), n, vp(g), vp(loss), None), "grad")
+    torch.cuda.synchronize()
+    ref_loss, ref_g = mlp.loss_grad(p.astype(np.float64), X, T)
+    assert abs(loss.item() / ref_loss - 1.0) < 2e-3
+    got = g.cpu().numpy()
+    assert np.linalg.norm(got - ref_g) <= 5e-3 * np.linalg.norm(ref_g)
+    assert np.abs(got - ref_g).max() <= 2e-2 * np.abs(ref_g).max()
+    assert (buf[:shift] == 7.0).all() and (buf[shift + mlp.NPARAM:] == 7.0).all()
