@@ -48,6 +48,18 @@ int cuda_err(cudaError_t e, const char *where)
 
 using namespace pt_internal;
 
+/* SMs of the device that is current at the first call. */
+int pt_coop_sms()
+{
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n < 1 ? 1 : n;
+    }();
+    return sms;
+}
+
 extern "C" const char *pt_last_error(void) { return g_err; }
 extern "C" int32_t pt_abi_version(void) { return PT_ABI_VERSION; }
 
@@ -298,8 +310,23 @@ void attach_fields(const pt_fields *f, PtRun &R)
            : f->precision == PT_PREC_FP32 ? nbk * 512                 /* compact bricks */
            : f->nodes;
     R.oob = f->scratch + 2;
+}
+
+void attach_hand(const pt_fields *fc, PtRun &R, cudaStream_t s)
+{
+    pt_fields *f = const_cast<pt_fields *>(fc);
+    if (R.np <= pt_coop_max()) return;
+    if (!f->hand) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone ||
+            cudaMalloc(&f->hand, (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8) != cudaSuccess) {
+            f->hand = nullptr;
+            (void)cudaGetLastError();          /* the run goes without */
+            return;
+        }
+    }
     R.hand.ctl = f->scratch + 3;
-    R.hand.rec = reinterpret_cast<double *>(f->scratch + 32);
+    R.hand.rec = f->hand;
 }
 
 int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
@@ -324,6 +351,8 @@ int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
         if (R.minb == 0) R.minb = (t & 0xff) ? (t & 0xff) : PT_MINB_DEFAULT;
         if (R.block == 0) R.block = (t >> 8) ? (t >> 8) : PT_BLOCK_DEFAULT;
     }
+
+    attach_hand(f, R, s);
 
     cudaError_t e;
     if (d_status && np > 0) {
@@ -385,6 +414,7 @@ extern "C" int pt_autotune(int32_t method, int64_t np, int32_t m, const pt_field
     attach_fields(f, R);
     R.queue = f->scratch;
     R.flags = reinterpret_cast<int32_t *>(f->scratch + 1);
+    attach_hand(f, R, s);
     if (!windowed && !(opt && opt->max_steps > 0)) R.max_steps = 32;
     /* One trial of variant (minb, block index) on fresh copies of the states. */
     auto trial = [&](int minb, int bi, bool keep) {

@@ -337,6 +337,17 @@ struct PtLaunch {
     cudaStream_t stream;
 };
 
+/* Particles up to which a run goes to the eight-lane machine from the start,
+ * PT_COOP_PER_SM per SM.  Exact build, one against eight lanes per particle:
+ * 1,024 particles DOP853 11.8 / 3.6 ms, RK5 10.1 / 3.4 ms; 9,728 11.8 / 7.7
+ * and 10.6 / 7.2; 12,160 (80 per SM) 11.8 / 9.4 and 10.6 / 8.6, where one lane
+ * with hand-over takes 10.7 and 8.9; 16,384 11.8 / 12.2 and 10.7 / 11.4. */
+#ifndef PT_COOP_PER_SM
+#define PT_COOP_PER_SM 80
+#endif
+int pt_coop_sms();
+inline int64_t pt_coop_max() { return (int64_t)PT_COOP_PER_SM * pt_coop_sms(); }
+
 #define PT_DECLARE_FP64_LAUNCHERS(sfx)                                            \
     cudaError_t pt_launch_rk5_##sfx(const PtRun &P, int nc, cudaStream_t s);     \
     cudaError_t pt_launch_dp853_##sfx(const PtRun &P, int nc, cudaStream_t s);   \

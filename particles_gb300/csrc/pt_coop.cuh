@@ -541,32 +541,13 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
 }
 #undef PT_Q
 
-/* Particles up to which a run goes to the eight-lane machine from the start,
- * per SM.  Exact build, one against eight lanes per particle: 1,024 particles
- * DOP853 11.8 / 3.6 ms, RK5 10.1 / 3.4 ms; 9,728 11.8 / 7.7 and 10.6 / 7.2;
- * 12,160 (80 per SM) 11.8 / 9.4 and 10.6 / 8.6, where one lane with
- * hand-over takes 10.7 and 8.9; 16,384 11.8 / 12.2 and 10.7 / 11.4. */
-#ifndef PT_COOP_PER_SM
-#define PT_COOP_PER_SM 80
-#endif
-inline int coop_sms()
-{
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n < 1 ? 1 : n;
-    }();
-    return sms;
-}
-
 /* Launch of an eight-lane kernel for n particles at most (n < 0: unknown, fill
  * the GPU).  Runs of under four groups per scheduler take one-warp blocks,
  * which spread over all SMs. */
 template <int METHOD, class EV, class KERN, class... Args>
 cudaError_t launch_coop(KERN kern, int64_t n, bool learn, cudaStream_t s, Args... args)
 {
-    const int sms = coop_sms();
+    const int sms = pt_coop_sms();
     const int block = (n >= 0 && n < 16 * (int64_t)sms) ? 32 : 128;
     const int64_t full = (int64_t)sms * 3;
     int64_t grid = n < 0 ? full : (n * kGroup + block - 1) / block;

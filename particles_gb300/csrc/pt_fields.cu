@@ -290,7 +290,7 @@ static int fields_create_impl(const int32_t dm[3], const double *uu, const doubl
     for (int i = 0; i < 3; ++i) f->nb[i] = (dm[i] + 7) / 8;
     f->nodes = nn;
     PT_CU(cudaGetDevice(&f->device));
-    PT_CU(cudaMalloc(&f->scratch, 256 + (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8));
+    PT_CU(cudaMalloc(&f->scratch, 256));
     PT_CU(cudaMemset(f->scratch, 0, 256));
     if (precision == PT_PREC_BF16) {
         const int64_t nbk = (int64_t)f->nb[0] * f->nb[1] * f->nb[2];
@@ -380,6 +380,7 @@ extern "C" int pt_fields_destroy(pt_fields *f)
     cudaFree(f->rec16);
     cudaFree(f->bscale);
     cudaFree(f->scratch);
+    cudaFree(f->hand);
     cudaFree(f->ws);
     cudaFree(f->pack);
     cudaFreeHost(f->hst);

@@ -483,7 +483,7 @@ cudaError_t launch_ens1(const PtRun *tab, int nmem, int block, int64_t ntot, cud
 {
     static int cache[2] = { -1, 1 };
     const int smem = pt_sm::smem_bytes<METHOD>(block, false);
-    const int64_t few = (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+    const int64_t few = pt_coop_max();
     return pt_sm::launch_persistent(k_ensemble<METHOD, NC, MINB>, block, smem,
                                     pt_sm::smem_bytes<METHOD>(PT_BLOCK_MAX, false), cache, ntot, s,
                                     tab, nmem, few);
@@ -505,7 +505,7 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
      * are launched, and the one that is not to take the queue finds nothing */
     if (e == cudaSuccess && ntot > 0)
         e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_ensemble_coop<METHOD, NC>, -1, false, s, tab, nmem,
-                                                    (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
+                                                    pt_coop_max());
     return e;
 }
 
@@ -524,7 +524,7 @@ cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
     if (P.rec) return launch_v<METHOD, NC, true>(P, s);
-    const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+    const bool few = P.np <= pt_coop_max();
     cudaError_t e = few ? cudaSuccess : P.mlp ? launch_v<METHOD, NC, true>(P, s) : launch_v<METHOD, NC, false>(P, s);
     if (e == cudaSuccess && (few || P.hand.ctl)) {
         if (P.mlp) e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC, true>, few ? P.np : -1, true, s, P, few);

@@ -45,7 +45,8 @@ struct pt_fields {
     int32_t nc16;               /* BF16 record width: 8 or 16 */
     int64_t bytes;
     unsigned long long *scratch;   /* [0] queue head, [1] flags (2 x int32), [2] out-of-range
-                                      count, [3..4] PtHand.ctl, [32..] PtHand.rec */
+                                      count, [3..4] PtHand.ctl */
+    double *hand;               /* PtHand.rec, allocated by the first run that hands over */
     unsigned char *ws;          /* host-buffer runs: device copies, reused across calls */
     size_t ws_bytes;
     unsigned char *pack;        /* host-buffer runs: the output rows a call wrote, packed */
@@ -69,6 +70,9 @@ int prepare_run(int32_t method, int64_t np, int32_t m, const RunShape &g, const 
                 const pt_options *opt, PtRun &R);
 /* The device pointers of a field handle in a run. */
 void attach_fields(const pt_fields *f, PtRun &R);
+/* The hand-over list of a run of R.np particles: none for runs that do not hand
+ * over, and where it would have to be allocated during a stream capture. */
+void attach_hand(const pt_fields *f, PtRun &R, cudaStream_t s);
 /* The kernel of the run's family (precision, method, record width). */
 cudaError_t launch_run(int32_t method, const pt_fields *f, const PtRun &R, cudaStream_t s);
 /* A run on device buffers: prepare, reset the queue and statuses, launch. */

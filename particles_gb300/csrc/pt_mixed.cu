@@ -461,7 +461,7 @@ cudaError_t launch_ens1(const PtRun *tab, int nmem, int block, int64_t ntot, cud
     return pt_sm::launch_persistent(k_ensemble_mixed<METHOD, EV, MINB>, block, smem,
                                     pt_sm::smem_bytes<METHOD>(PT_BLOCK_MAX, false), cache,
                                     ntot, s, tab, nmem,
-                                    (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
+                                    pt_coop_max());
 }
 
 template <int METHOD, class EV>
@@ -480,7 +480,7 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
      * are launched, and the one that is not to take the queue finds nothing */
     if (e == cudaSuccess && ntot > 0)
         e = pt_sm::launch_coop<METHOD, EV>(k_ensemble_coop_mixed<METHOD, EV>, -1, false, s, tab, nmem,
-                                           (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms());
+                                           pt_coop_max());
     return e;
 }
 
@@ -501,7 +501,7 @@ cudaError_t launch(const PtRun &P, cudaStream_t s)
     if (P.np <= 0) return cudaSuccess;
     if (LEARNABLE && P.rec) return launch_v<METHOD, EV, LEARNABLE>(P, s);
     const bool learn = LEARNABLE && P.mlp;
-    const bool few = P.np <= (int64_t)PT_COOP_PER_SM * pt_sm::coop_sms();
+    const bool few = P.np <= pt_coop_max();
     cudaError_t e = few ? cudaSuccess : learn ? launch_v<METHOD, EV, LEARNABLE>(P, s) : launch_v<METHOD, EV, false>(P, s);
     if (e == cudaSuccess && (few || P.hand.ctl)) {
         if (learn) e = pt_sm::launch_coop<METHOD, EV>(k_coop_mixed<METHOD, EV, LEARNABLE>, few ? P.np : -1, true, s, P, few);
