@@ -277,10 +277,15 @@ static int fields_create_impl(const int32_t dm[3], const double *uu, const doubl
         return set_err(PT_ERR_UNSUPPORTED, "pt_fields_create: precision not built%s");
 
     int rc = PT_OK;
+    const size_t bytes3 = (size_t)dm[0] * dm[1] * dm[2] * 3 * sizeof(double);
+    /* host arrays that the packing kernels can read in place: no copies */
+    if (!on_device)
+        on_device = host_direct(uu, bytes3, false) && host_direct(bb, bytes3, false) &&
+                    (!jj || host_direct(jj, bytes3, false));
     pt_fields *f = new pt_fields();
     double *d_uu = nullptr, *d_bb = nullptr, *d_jj = nullptr;
     const int64_t nn = (int64_t)dm[0] * dm[1] * dm[2];
-    const size_t plane3 = (size_t)nn * 3 * sizeof(double);
+    const size_t plane3 = bytes3;
     for (int i = 0; i < 3; ++i) f->dm[i] = dm[i];
     f->precision = precision;
     f->has_j = jj != nullptr;

@@ -83,6 +83,10 @@ int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f, const do
 int32_t pt_opt_threads_per_block(const pt_options *opt);
 /* pt_options.open_x_margin when the caller's struct has the field, else 0. */
 double pt_opt_open_x_margin(const pt_options *opt);
+/* Whether kernels may read (write: and write) the caller's host array in place:
+ * it is pinned, or the GPU shares the host's page tables and the array's pages
+ * are mapped (pt_hostio.cu). */
+bool host_direct(const void *p, size_t bytes, bool write);
 /* The launch variant pt_autotune chose for a kernel family (0: none). */
 std::atomic<int> &tuned_slot(int32_t method, const pt_fields *f, const PtRun &R);
 
