@@ -331,7 +331,7 @@ void attach_hand(const pt_fields *fc, PtRun &R, cudaStream_t s)
 
 int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
                     const double *params, const double *d_time, double *d_state, int64_t *d_cnt,
-                    int32_t *d_status, void *d_carry, const pt_options *opt, cudaStream_t s)
+                    int32_t *d_status, void *d_carry, const pt_options *opt, cudaStream_t s, bool fresh)
 {
     if (!f) return set_err(PT_ERR_ARG, "fields handle is NULL%s");
     if (np > 0 && (!d_time || !d_state || !d_cnt)) return set_err(PT_ERR_ARG, "NULL buffer%s");
@@ -344,6 +344,7 @@ int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
     R.cnt = d_cnt;
     R.status = d_status;
     R.carry = static_cast<unsigned char *>(d_carry);
+    R.fresh = fresh || !d_carry;
     R.queue = f->scratch;
     R.flags = reinterpret_cast<int32_t *>(f->scratch + 1);
     if (R.minb == 0 || R.block == 0) {
@@ -408,6 +409,7 @@ extern "C" int pt_autotune(int32_t method, int64_t np, int32_t m, const pt_field
     R.cnt = t_cnt;
     R.status = nullptr;
     R.carry = nullptr;
+    R.fresh = 1;
     R.order = nullptr;
     R.rec = t_rec;
     R.rec_cap = 0;

@@ -212,7 +212,7 @@ extern "C" int pt_integrate_fields(int32_t method, int64_t np, int32_t m, const 
             PT_CU(cudaMemsetAsync(d_carry, 0, crb, s));              /* every particle fresh */
         }
         PT_CU(cudaMemcpyAsync(d_nf0, d_n, (size_t)np * 8, cudaMemcpyDeviceToDevice, s));
-        rc = run_impl(method, np, m, f, params, d_time, d_state, d_cnt, d_status, d_carry, opt, s);
+        rc = run_impl(method, np, m, f, params, d_time, d_state, d_cnt, d_status, d_carry, opt, s, !h_carry);
         if (rc != PT_OK) goto done;
         double *staged = nullptr;
         unsigned long long *const d_total = reinterpret_cast<unsigned long long *>(d_off);

@@ -75,10 +75,11 @@ void attach_fields(const pt_fields *f, PtRun &R);
 void attach_hand(const pt_fields *f, PtRun &R, cudaStream_t s);
 /* The kernel of the run's family (precision, method, record width). */
 cudaError_t launch_run(int32_t method, const pt_fields *f, const PtRun &R, cudaStream_t s);
-/* A run on device buffers: prepare, reset the queue and statuses, launch. */
+/* A run on device buffers: prepare, reset the queue and statuses, launch.  fresh:
+ * the carry, if there is one, holds no started particle. */
 int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f, const double *params,
              const double *d_time, double *d_state, int64_t *d_cnt, int32_t *d_status,
-             void *d_carry, const pt_options *opt, cudaStream_t s);
+             void *d_carry, const pt_options *opt, cudaStream_t s, bool fresh = false);
 /* pt_options.threads_per_block when the caller's struct has the field, else 0. */
 int32_t pt_opt_threads_per_block(const pt_options *opt);
 /* pt_options.open_x_margin when the caller's struct has the field, else 0. */

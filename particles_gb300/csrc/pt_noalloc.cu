@@ -165,6 +165,7 @@ extern "C" int pt_integrate_device_noalloc(int32_t method, int64_t np, int32_t m
         R.cnt = d_cnt;
         R.status = d_status;
         R.carry = nullptr;
+        R.fresh = 1;
         R.queue = reinterpret_cast<unsigned long long *>(base);
         R.flags = reinterpret_cast<int32_t *>(base + sizeof(unsigned long long));
         R.oob = reinterpret_cast<unsigned long long *>(base + 2 * sizeof(unsigned long long));
