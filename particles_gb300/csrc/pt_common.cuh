@@ -245,6 +245,28 @@ __device__ __forceinline__ void pt_axis_exact(double x, int32_t d, int32_t mask,
     }
 }
 
+/* The IEEE division for quotients and reciprocals outside the fast forms'
+ * domains, out of line: inlined at every use its own slow path makes the
+ * compiler spill around code that physical states never reach. */
+static __device__ __noinline__ double pt_div_cold(double a, double b) { return a / b; }
+
+/* 1 / b correctly rounded: the hardware's approximation (20 bits and more),
+ * two Newton steps to within an ulp, and a third that rounds correctly unless
+ * the significand of b is all ones (P. Markstein, IBM J. Res. Develop. 34(1),
+ * 1990, for fused multiply-add).  That case, and b whose reciprocal's steps could
+ * leave the normal range (also zero, infinity, NaN), take the division.  Six
+ * FP64 operations against about nine. */
+__device__ __forceinline__ double pt_recip(double b)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(b), e = (hi >> 20) & 0x7ffu;
+    if (e - 24u > 1998u || ((hi & 0xfffffu) == 0xfffffu && __double2loint(b) == -1)) return pt_div_cold(1.0, b);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(fma(-b, y, 1.0), y, y);
+    y = fma(fma(-b, y, 1.0), y, y);
+    return fma(fma(-b, y, 1.0), y, y);
+}
+
 /* a / b correctly rounded from y = RN(1/b) (Markstein's quotient correction,
  * P. Markstein, IBM J. Res. Develop. 34(1), 1990): q0 = RN(a y) is within an
  * ulp of a / b, so the remainder r = a - b q0 is exact in one FMA and
@@ -260,7 +282,7 @@ __device__ __forceinline__ double pt_qdiv(double a, double b, double y)
     const double q0 = pt_fmul(a, y);
     const uint32_t e = (uint32_t)((unsigned long long)__double_as_longlong(q0) >> 52) & 0x7ffu;
     const uint32_t ea = (uint32_t)((unsigned long long)__double_as_longlong(a) >> 52) & 0x7ffu;
-    if (e - 63u > 1920u || ea < 116u) return a / b;
+    if (e - 63u > 1920u || ea < 116u) return pt_div_cold(a, b);
     const double r = fma(-b, q0, a);
     return fma(r, y, q0);
 }

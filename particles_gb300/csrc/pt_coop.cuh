@@ -259,7 +259,7 @@ __device__ __forceinline__ double coop_finish(const PtRun &P, const Group &G, co
         const PtR e5 = PtR(ER01) * K(0) + PtR(ER06) * K(5) + PtR(ER07) * K(6) + PtR(ER08) * K(7)
                      + PtR(ER09) * K(8) + PtR(ER10) * K(9) + PtR(ER11) * K(1) + PtR(ER12) * K(2);
 #ifdef PT_EXACT
-        const double ysr = 1.0 / sr;
+        const double ysr = pt_recip(sr);
         const PtR q3 = pt_qdiv(e3, sr, ysr), q5 = pt_qdiv(e5, sr, ysr);
         const double t3 = q3 * q3, t5 = q5 * q5;       /* squared before they are handed round */
 #else

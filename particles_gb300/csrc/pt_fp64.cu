@@ -215,7 +215,7 @@ struct EvalF64 {
          * reciprocal each: bit-identical to the divisions (pt_qdiv) */
         const PtR u0 = s[3], u1 = s[4], u2 = s[5];
         const double g = sqrt(u0 * u0 + u1 * u1 + u2 * u2 + 1.0);
-        const double yg = 1.0 / g;
+        const double yg = pt_recip(g);
         const PtR v0 = pt_qdiv(s[3], g, yg), v1 = pt_qdiv(s[4], g, yg), v2 = pt_qdiv(s[5], g, yg);
         a[0] = pt_qdiv(v0, P.vun, P.inv_vun);
         a[1] = pt_qdiv(v1, P.vun, P.inv_vun);
@@ -309,7 +309,7 @@ struct CoopF64 : EvalF64<NC> {
 #ifdef PT_EXACT
         const double ss = pt_fmul(s, s);
         const double g = sqrt(PtR(G.get(ss, 3)) + G.get(ss, 4) + G.get(ss, 5) + 1.0);
-        const double vel = pt_qdiv(s, g, 1.0 / g);
+        const double vel = pt_qdiv(s, g, pt_recip(g));
 #else
         const double s3 = G.get(s, 3), s4 = G.get(s, 4), s5 = G.get(s, 5);
         const double ig = pt_sm::pt_rsqrt(fma(s3, s3, fma(s4, s4, fma(s5, s5, 1.0))));
@@ -374,7 +374,7 @@ struct CoopF64 : EvalF64<NC> {
         if (pos) {
             const uint32_t e = (uint32_t)((unsigned long long)__double_as_longlong(p1) >> 52) & 0x7ffu;
             const uint32_t ea = (uint32_t)((unsigned long long)__double_as_longlong(vp) >> 52) & 0x7ffu;
-            if (e - 63u > 1920u || ea < 116u) a = vp / P.vun;  /* pt_qdiv's excluded quotients */
+            if (e - 63u > 1920u || ea < 116u) a = pt_div_cold(vp, P.vun);  /* pt_qdiv's excluded quotients */
         }
         double f = a;
         if (NV == 9) {

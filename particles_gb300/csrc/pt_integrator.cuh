@@ -236,7 +236,7 @@ __device__ __forceinline__ double dti_finish(const PtRun &P, int iord, const dou
      * operations weigh as much as an RK5 attempt */
     double sr[6], y[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) { sr[i] = P.atol + P.rtol * fabs(si[i]); y[i] = 1.0 / sr[i]; }
+    for (int i = 0; i < 6; ++i) { sr[i] = P.atol + P.rtol * fabs(si[i]); y[i] = pt_recip(sr[i]); }
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) { const double q = pt_qdiv(si[i], sr[i], y[i]); s0 = s0 + q * q; }
@@ -433,7 +433,7 @@ __device__ __forceinline__ double finish_attempt(const PtRun &P, const KRows &K,
          * shared by the two sums: bit-identical to the divisions (pt_qdiv) */
         double ysr[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) ysr[c] = 1.0 / sr[c];
+        for (int c = 0; c < 6; ++c) ysr[c] = pt_recip(sr[c]);
 #define PT_OVER_SR(e, c) pt_qdiv((e), sr[c], ysr[c])
 #endif
 #pragma unroll

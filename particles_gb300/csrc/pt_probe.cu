@@ -48,14 +48,14 @@ __global__ void k_face_cap(const PtRun P, int64_t n, const double *si, const dou
     }
 }
 
-/* pt_qdiv next to the IEEE division: out[2i] = pt_qdiv(a, b, 1 / b),
+/* pt_qdiv next to the IEEE division: out[2i] = pt_qdiv(a, b, pt_recip(b)),
  * out[2i + 1] = a / b. */
 __global__ void k_qdiv(int64_t n, const double *a, const double *b, double *out)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const double x = a[i], y = b[i];
-        out[2 * i] = pt_qdiv(x, y, 1.0 / y);
+        out[2 * i] = pt_qdiv(x, y, pt_recip(y));
         out[2 * i + 1] = x / y;
     }
 }
