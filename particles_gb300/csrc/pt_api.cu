@@ -327,6 +327,7 @@ void attach_hand(const pt_fields *fc, PtRun &R, cudaStream_t s)
     }
     R.hand.ctl = f->scratch + 3;
     R.hand.rec = f->hand;
+    R.hand.lanes = pt_hand_lanes(R.np, f->precision);
 }
 
 int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,

@@ -26,20 +26,13 @@
  * records, ctl[1] is the head they are taken from; a record holds a particle
  * between two attempts. */
 #define PT_HAND_WORDS 22
-/* 16 warps on each of 152 SMs with PT_HAND_LANES particles each; a warp that
- * finds the list full keeps its particles */
+/* 16 warps on each of 152 SMs with 12 particles each; a warp that finds the list
+ * full keeps its particles */
 #define PT_HAND_CAP 32768
-/* Lanes a warp still has at work when it hands over.  One lane per particle
- * costs a scheduler ~2,500 FP64 slots per attempt for up to 32 particles,
- * eight lanes ~900 for 4: equal at about 11.  Measured, exact build, 65,536
- * particles, never / 4 / 8 / 12 / 16 / 24: DOP853 25.3 / 21.9 / 20.2 / 20.0 /
- * 26.8 / 29.2 ms, RK5 21.4 / 18.3 / 17.3 / 17.2 / 23.9 / 26.0 ms. */
-#ifndef PT_HAND_LANES
-#define PT_HAND_LANES 12
-#endif
 struct PtHand {
     unsigned long long *ctl;  /* 2 words, zeroed before a launch; NULL: no hand-over */
     double *rec;              /* PT_HAND_WORDS words per record */
+    int lanes;                /* lanes a warp still has at work when it hands over */
 };
 
 /* Everything a particle-integration kernel reads, by value in the launch. */
@@ -370,6 +363,21 @@ struct PtLaunch {
 #endif
 int pt_coop_sms();
 inline int64_t pt_coop_max() { return (int64_t)PT_COOP_PER_SM * pt_coop_sms(); }
+/* Lanes a warp still has at work when it hands over.  One lane per particle
+ * costs a scheduler ~2,400 FP64 slots per DOP853 attempt for up to 32 particles,
+ * eight lanes ~900 for 4: equal at about 11 where the schedulers are full.
+ * Exact build, 65,536 particles, never / 4 / 8 / 12 / 16 / 24: DOP853 25.3 / 21.9
+ * / 20.2 / 20.0 / 26.8 / 29.2 ms, RK5 21.4 / 18.3 / 17.3 / 17.2 / 23.9 / 26.0.
+ * Where one warp per scheduler holds the whole run, the eight-lane machine's
+ * shorter attempt counts instead.  12 / 16 / 20 / 24 lanes: exact DOP853 16,384
+ * particles 9.5 / 8.9 / 8.9 / 8.9 ms, 20,001 10.6 / 10.1 / 10.1 / 10.3, 32,768
+ * 11.5 / 11.4 / 11.9 / 12.3; FP32 DOP853 16,384 9.5 / 8.8 / 8.5 / 8.2, 32,768
+ * 10.8 / 10.5 / 10.3 / 9.9. */
+inline int pt_hand_lanes(int64_t np, int precision)
+{
+    const bool mixed = precision == PT_PREC_FP32 || precision == PT_PREC_BF16;
+    return np <= (mixed ? 240 : 160) * (int64_t)pt_coop_sms() ? (mixed ? 24 : 20) : 12;
+}
 
 #define PT_DECLARE_FP64_LAUNCHERS(sfx)                                            \
     cudaError_t pt_launch_rk5_##sfx(const PtRun &P, int nc, cudaStream_t s);     \

@@ -938,7 +938,7 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                 if (!__any_sync(0xffffffffu, !drained)) break;
                 continue;                                               /* j stays 0 */
             }
-            if (HAND && __popc(act) <= PT_HAND_LANES && __any_sync(0xffffffffu, drained)) {
+            if (HAND && __popc(act) <= MB.q(0).hand.lanes && __any_sync(0xffffffffu, drained)) {
                 const PtHand H = MB.q(0).hand;
                 if (H.ctl && !(LEARN && MB.q(0).rec)) {   /* recording keeps its pending records */
                     const int lane = threadIdx.x & 31;
