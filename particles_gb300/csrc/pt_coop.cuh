@@ -216,18 +216,37 @@ __device__ __forceinline__ void coop_stage(int j, const KOwn &K, double si, doub
             coop_step<DELTA>(PtR(dt) * S.a[0], K(0), si, ss, dl);
         } else {
             PtR acc = PtR(S.a[0]) * K(S.r[0]);
-            for (int i = 1; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i]);
+            /* the next term's coefficient and row are on their way during this one */
+            double a = S.a[1], k = K(S.r[1]);
+            for (int i = 1; i < S.n; ++i) {
+                const double an = S.a[i + 1], kn = K(S.r[i + 1]);
+                acc = acc + PtR(a) * k;
+                a = an;
+                k = kn;
+            }
             coop_step<DELTA>(dt, acc, si, ss, dl);
         }
     } else {
         const Stage &S = kCk[j];
         if (DELTA) {
             double acc = S.a[0] * K(S.r[0]);
-            for (int i = 1; i < S.n; ++i) acc = acc + S.a[i] * K(S.r[i]);
+            double a = S.a[1], k = K(S.r[1]);
+            for (int i = 1; i < S.n; ++i) {
+                const double an = S.a[i + 1], kn = K(S.r[i + 1]);
+                acc = acc + a * k;
+                a = an;
+                k = kn;
+            }
             dl = acc;
         } else {
             PtR acc = si;
-            for (int i = 0; i < S.n; ++i) acc = acc + PtR(S.a[i]) * K(S.r[i]);
+            double a = S.a[0], k = K(S.r[0]);
+            for (int i = 0; i < S.n; ++i) {
+                const double an = S.a[i + 1], kn = K(S.r[i + 1]);
+                acc = acc + PtR(a) * k;
+                a = an;
+                k = kn;
+            }
             ss = acc;
         }
     }

@@ -67,8 +67,8 @@ using namespace pt_tab;
  * with coefficients a[], and f(stage) is stored into row dst. */
 struct Stage {
     int n, dst;
-    double a[9];
-    int r[9];
+    double a[10];          /* one more than the longest sum: pt_coop.cuh reads a term ahead */
+    int r[10];
 };
 
 /* DOP853 (integrations.F90:365-416): k rows 0..9 as in the reference's
