@@ -1410,7 +1410,11 @@ def main():
                   "bf16": "f64 step machine, f32 gather/force, bf16 field store"}[args.precision],
         "data": "synthetic (seeded fields and particles)",
         "config": workload_config(cfg, npart, window, args),
-        "wall_s_timed": wall, "gpu_launches": args.steps, "stopped_particles": stopped,
+        # a window is k_integrate and the k_coop that takes its last particles
+        # (a run of at most 80 particles per SM is k_coop alone)
+        "wall_s_timed": wall, "stopped_particles": stopped,
+        "gpu_launches": args.steps * (2 if npart > 80 * torch.cuda.get_device_properties(dev)
+                                      .multi_processor_count else 1),
         "rejected_fraction": float(dcnt_tot[2] / max(dcnt_tot[0], 1)),
         "attempts_per_s": float(dcnt_tot[0]) / elapsed,
         "particle_gyroperiods_per_s": world * npart * window * args.steps / elapsed,
