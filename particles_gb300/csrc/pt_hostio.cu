@@ -34,7 +34,16 @@ bool host_direct(const void *p, size_t bytes, bool write)
         (void)cudaGetLastError();
         return false;
     }
-    if (a.type == cudaMemoryTypeHost) return a.devicePointer == p;
+    if (a.type == cudaMemoryTypeHost) {
+        /* pinned to its end, not in its first pages only */
+        const char *end = static_cast<const char *>(p) + bytes - 1;
+        cudaPointerAttributes z;
+        if (cudaPointerGetAttributes(&z, end) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        return a.devicePointer == p && z.type == cudaMemoryTypeHost && z.devicePointer == end;
+    }
     if (a.type != cudaMemoryTypeUnregistered) return false;
     int dev = 0, shared = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

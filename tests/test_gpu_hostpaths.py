@@ -47,3 +47,26 @@ def test_host_rows_bitwise(cuda, oracle_lib, nsteps, align, pinned):
     s2 = host(prob["state"])
     _, c2, _ = integrate("rk5", prob["params"], tg, host(uu), host(bb), s2)
     assert np.array_equal(c2, co) and np.array_equal(s2, so)
+
+
+def test_state_pinned_in_part(cuda, oracle_lib):
+    """Only the first pages of the state are registered with the GPU."""
+    import mmap
+    import oracle
+    from particles_gb300 import integrate
+    npart = 2 * mmap.PAGESIZE // 64                         # six rows each: twelve pages
+    prob = small_problem("rk5", n=10, npart=npart, periods=0.02, seed=92, nsteps=5, tol=1e-6)
+    uu, bb = prob["fields"]
+    so, co, _ = oracle.integrate("rk5", prob["params"], prob["time"], uu, bb, prob["state"].copy())
+    a = prob["state"]
+    flat = np.zeros(a.size + mmap.PAGESIZE // 8)
+    off = (-flat.ctypes.data % mmap.PAGESIZE) // 8
+    s = flat[off:off + a.size].reshape(a.shape)
+    s[:] = a
+    rt = cuda.cuda.cudart()
+    assert int(rt.cudaHostRegister(s.ctypes.data, mmap.PAGESIZE, 0)) == 0
+    try:
+        _, cnt, _ = integrate("rk5", prob["params"], prob["time"], uu, bb, s)
+    finally:
+        rt.cudaHostUnregister(s.ctypes.data)
+    assert np.array_equal(cnt, co) and np.array_equal(s, so)
