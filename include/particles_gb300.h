@@ -413,6 +413,12 @@ int pt_debug_face_params(int32_t method, float skip, float over);
  * straight path + overshoot). */
 int pt_debug_face_cap(const pt_fields *f, int32_t method, int64_t n, const double params[17],
                       const double *d_si, const double *d_h, double *d_out, void *stream);
+/* For tests, in the calling thread only: a run (or an ensemble's window) of
+ * more than `limit` particles starts on one lane per particle, a smaller one on
+ * eight, and `hand_cap` particles at most pass from one machine to the other
+ * where a run ends (0: none); -1: the library's own values.  No particle's
+ * result depends on either.  Returns the limit now in force. */
+int64_t pt_debug_machines(int64_t limit, int32_t hand_cap);
 int pt_debug_accel(const pt_fields *f, int64_t n, const double params[17],
                    const double *d_vec, double *d_acc, void *stream);
 

@@ -60,6 +60,24 @@ int pt_coop_sms()
     return sms;
 }
 
+/* pt_debug_machines of the calling thread; -1: the library's own */
+static thread_local int64_t g_coop_limit = -1;
+static thread_local int g_hand_cap = -1;
+
+int64_t pt_coop_max()
+{
+    return g_coop_limit >= 0 ? g_coop_limit : (int64_t)PT_COOP_PER_SM * pt_coop_sms();
+}
+
+int pt_hand_cap() { return g_hand_cap >= 0 ? g_hand_cap : PT_HAND_CAP; }
+
+extern "C" int64_t pt_debug_machines(int64_t limit, int32_t hand_cap)
+{
+    g_coop_limit = limit < 0 ? -1 : limit;
+    g_hand_cap = hand_cap < 0 || hand_cap > PT_HAND_CAP ? -1 : hand_cap;
+    return pt_coop_max();
+}
+
 extern "C" const char *pt_last_error(void) { return g_err; }
 extern "C" int32_t pt_abi_version(void) { return PT_ABI_VERSION; }
 
@@ -328,6 +346,7 @@ void attach_hand(const pt_fields *fc, PtRun &R, cudaStream_t s)
     R.hand.ctl = f->scratch + 3;
     R.hand.rec = f->hand;
     R.hand.lanes = pt_hand_lanes(R.np, f->precision);
+    R.hand.cap = pt_hand_cap();
 }
 
 int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,

@@ -19,6 +19,7 @@
 
 #include "../../include/particles_gb300.h"
 #include "pt_detmath.h"
+#include "pt_hand.h"
 #include "pt_smul.h"
 
 /* Particles handed from the lane-per-particle machine to the eight-lane one
@@ -26,13 +27,15 @@
  * records, ctl[1] is the head they are taken from; a record holds a particle
  * between two attempts. */
 #define PT_HAND_WORDS 22
-/* 16 warps on each of 152 SMs with 12 particles each; a warp that finds the list
- * full keeps its particles */
+/* 16 warps on each of 152 SMs (the kernels' register counts allow no more) with
+ * 12 particles each, or the warps of 240 particles per SM with 24 each; a warp
+ * whose particles do not fit any more keeps them */
 #define PT_HAND_CAP 32768
 struct PtHand {
     unsigned long long *ctl;  /* 2 words, zeroed before a launch; NULL: no hand-over */
     double *rec;              /* PT_HAND_WORDS words per record */
     int lanes;                /* lanes a warp still has at work when it hands over */
+    int cap;                  /* records that fit */
 };
 
 /* Everything a particle-integration kernel reads, by value in the launch. */
@@ -362,7 +365,8 @@ struct PtLaunch {
 #define PT_COOP_PER_SM 80
 #endif
 int pt_coop_sms();
-inline int64_t pt_coop_max() { return (int64_t)PT_COOP_PER_SM * pt_coop_sms(); }
+int64_t pt_coop_max();                /* particles; pt_debug_machines may change both */
+int pt_hand_cap();                    /* records of a hand-over list */
 /* Lanes a warp still has at work when it hands over.  One lane per particle
  * costs a scheduler ~2,400 FP64 slots per DOP853 attempt for up to 32 particles,
  * eight lanes ~900 for 4: equal at about 11 where the schedulers are full.

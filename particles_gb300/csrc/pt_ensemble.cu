@@ -313,6 +313,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
     }
     e->hand.rec = reinterpret_cast<double *>(e->hand.ctl + 32);
     e->hand.lanes = pt_hand_lanes(ntot, prec);
+    e->hand.cap = pt_hand_cap();
     int64_t off = 0;
     for (int k = 0; k < nmembers; ++k) {
         const pt_member &M = members[k];

@@ -684,7 +684,7 @@ template <> struct Members<true> {
     __device__ __forceinline__ int count() const { return n; }
 };
 
-/* HAND: when the queue has run dry and at most kHandLanes lanes of a warp
+/* HAND: when the queue has run dry and at most PtHand.lanes lanes of a warp
  * still integrate, their particles go to the hand-over list. */
 template <int METHOD, class EV, bool LEARN, bool ENS = false, bool HAND = false>
 __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
@@ -943,14 +943,17 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                 if (H.ctl && !(LEARN && MB.q(0).rec)) {   /* recording keeps its pending records */
                     const int lane = threadIdx.x & 31;
                     unsigned long long at = 0;
-                    if (lane == 0) at = atomicAdd(H.ctl, (unsigned long long)__popc(act));
+                    if (lane == 0)
+                        at = pt_hand_reserve(*(volatile unsigned long long *)H.ctl, __popc(act), H.cap,
+                                             [&](unsigned long long e, unsigned long long w) {
+                                                 return atomicCAS(H.ctl, e, w);
+                                             });
                     at = __shfl_sync(0xffffffffu, at, 0);
-                    if (at + __popc(act) <= PT_HAND_CAP) {
+                    if (at < (unsigned long long)H.cap) {
                         at += __popc(act & ((1u << lane) - 1u));
                         if (active) lane_hand<METHOD>(H.rec + at * PT_HAND_WORDS, K, L, si, t_start, mi);
                         break;
                     }
-                    if (lane == 0) atomicAdd(H.ctl, 0ULL - (unsigned long long)__popc(act));
                 }
             }
         }
