@@ -330,18 +330,24 @@ void attach_fields(const pt_fields *f, PtRun &R)
     R.oob = f->scratch + 2;
 }
 
-void attach_hand(const pt_fields *fc, PtRun &R, cudaStream_t s)
+void attach_hand(const pt_fields *fc, PtRun &R)
 {
     pt_fields *f = const_cast<pt_fields *>(fc);
     if (R.np <= pt_coop_max()) return;
     if (!f->hand) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone ||
-            cudaMalloc(&f->hand, (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8) != cudaSuccess) {
-            f->hand = nullptr;
-            (void)cudaGetLastError();          /* the run goes without */
-            return;
+        /* In the default mode of a stream capture, here or in another thread, an
+         * allocation invalidates the capture, be it of another stream than this
+         * run's.  It is no part of any graph, so the relaxed mode fits. */
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e == cudaSuccess) {
+            e = cudaMalloc(&f->hand, (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8);
+            const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) f->hand = nullptr;
+            else e = back;
         }
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        if (!f->hand) return;                  /* the run goes without */
     }
     R.hand.ctl = f->scratch + 3;
     R.hand.rec = f->hand;
@@ -373,7 +379,7 @@ int run_impl(int32_t method, int64_t np, int32_t m, const pt_fields *f,
         if (R.block == 0) R.block = (t >> 8) ? (t >> 8) : PT_BLOCK_DEFAULT;
     }
 
-    attach_hand(f, R, s);
+    attach_hand(f, R);
 
     cudaError_t e;
     if (d_status && np > 0) {
@@ -436,7 +442,7 @@ extern "C" int pt_autotune(int32_t method, int64_t np, int32_t m, const pt_field
     attach_fields(f, R);
     R.queue = f->scratch;
     R.flags = reinterpret_cast<int32_t *>(f->scratch + 1);
-    attach_hand(f, R, s);
+    attach_hand(f, R);
     if (!windowed && !(opt && opt->max_steps > 0)) R.max_steps = 32;
     /* One trial of variant (minb, block index) on fresh copies of the states. */
     auto trial = [&](int minb, int bi, bool keep) {

@@ -71,8 +71,8 @@ int prepare_run(int32_t method, int64_t np, int32_t m, const RunShape &g, const 
 /* The device pointers of a field handle in a run. */
 void attach_fields(const pt_fields *f, PtRun &R);
 /* The hand-over list of a run of R.np particles: none for runs that do not hand
- * over, and where it would have to be allocated during a stream capture. */
-void attach_hand(const pt_fields *f, PtRun &R, cudaStream_t s);
+ * over, and where there is no memory for it. */
+void attach_hand(const pt_fields *f, PtRun &R);
 /* The kernel of the run's family (precision, method, record width). */
 cudaError_t launch_run(int32_t method, const pt_fields *f, const PtRun &R, cudaStream_t s);
 /* A run on device buffers: prepare, reset the queue and statuses, launch.  fresh:

@@ -1,0 +1,50 @@
+"""What a launch may do besides launching."""
+import pytest
+
+from conftest import small_problem
+
+pytestmark = pytest.mark.gpu
+
+
+def _big(torch, seed):
+    few = 80 * torch.cuda.get_device_properties(0).multi_processor_count
+    return small_problem("dop853", n=12, npart=few + 1, periods=0.03, seed=seed, nsteps=3)
+
+
+def _buffers(torch, prob):
+    npart = prob["state"].shape[0]
+    return dict(time=torch.tensor(prob["time"], device="cuda"), state=torch.tensor(prob["state"], device="cuda"),
+                cnt=torch.zeros((npart, 3), dtype=torch.int64, device="cuda"))
+
+
+def _run(f, prob, b, stream=0):
+    f.run_device("dop853", prob["params"], b["time"], b["state"], b["cnt"], stream=stream)
+
+
+@pytest.mark.parametrize("captured", ["another_stream", "its_own_stream"])
+def test_first_large_run_of_a_handle_during_a_capture(cuda, captured):
+    """A capture in the default (global) mode survives the first run of a handle
+    that is large enough to hand particles over, whichever stream that run is on."""
+    torch = cuda
+    from particles_gb300 import Fields
+    prob = _big(torch, 61)
+    uu, bb = prob["fields"]
+    ref = _buffers(torch, prob)
+    _run(Fields(uu, bb), prob, ref)                       # loads the kernels; the results to compare with
+    f, b = Fields(uu, bb), _buffers(torch, prob)
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+    x = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        g.capture_begin(capture_error_mode="global")
+        x.add_(1.0)
+        _run(f, prob, b, side.cuda_stream if captured == "its_own_stream" else other.cuda_stream)
+        g.capture_end()
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert f.run_check() == 0
+    assert x.tolist() == [1.0] * 8
+    assert torch.equal(b["cnt"], ref["cnt"])
+    assert torch.equal(b["state"].view(torch.int64), ref["state"].view(torch.int64))
