@@ -397,6 +397,10 @@ inline int pt_hand_lanes(int64_t np, int precision)
 PT_DECLARE_FP64_LAUNCHERS(exact)
 PT_DECLARE_FP64_LAUNCHERS(fma)
 
+/* Readies the exact kernels of a method for later runs without options (NC = 6). */
+cudaError_t pt_ready_rk5(const PtRun &P, cudaStream_t s);
+cudaError_t pt_ready_dp853(const PtRun &P, cudaStream_t s);
+
 cudaError_t pt_launch_rk5_mixed(const PtRun &P, int nc, cudaStream_t s);
 cudaError_t pt_launch_rk5_ens_mixed(const PtRun *tab, int nmem, int nc, int minb, int block,
                                     int64_t ntot, cudaStream_t s);

@@ -533,6 +533,19 @@ cudaError_t launch(const PtRun &P, cudaStream_t s)
     return e;
 }
 
+#ifdef PT_EXACT
+/* Both kernels of a run without options, launched on no particles: lazy loading
+ * and what the driver allocates for a kernel's first launch are over then. */
+template <int METHOD>
+cudaError_t ready(PtRun P, cudaStream_t s)
+{
+    P.np = 0;
+    cudaError_t e = launch_v<METHOD, 6, false>(P, s);
+    if (e == cudaSuccess) e = pt_sm::launch_coop<METHOD, CoopF64<6>>(k_coop<METHOD, 6, false>, 0, false, s, P, true);
+    return e;
+}
+#endif
+
 }  // namespace
 
 /* PT_PART splits the launchers over two translation units (1: RK5 and the
@@ -542,6 +555,10 @@ cudaError_t PT_NAME(pt_launch_rk5)(const PtRun &P, int nc, cudaStream_t s)
 {
     return nc == 10 ? launch<PT_METHOD_RK5, 10>(P, s) : launch<PT_METHOD_RK5, 6>(P, s);
 }
+
+#ifdef PT_EXACT
+cudaError_t pt_ready_rk5(const PtRun &P, cudaStream_t s) { return ready<PT_METHOD_RK5>(P, s); }
+#endif
 
 cudaError_t PT_NAME(pt_launch_rk5_ens)(const PtRun *tab, int nmem, int nc, int minb, int block,
                                        int64_t ntot, cudaStream_t s)
@@ -556,6 +573,10 @@ cudaError_t PT_NAME(pt_launch_dp853)(const PtRun &P, int nc, cudaStream_t s)
 {
     return nc == 10 ? launch<PT_METHOD_DOP853, 10>(P, s) : launch<PT_METHOD_DOP853, 6>(P, s);
 }
+
+#ifdef PT_EXACT
+cudaError_t pt_ready_dp853(const PtRun &P, cudaStream_t s) { return ready<PT_METHOD_DOP853>(P, s); }
+#endif
 
 cudaError_t PT_NAME(pt_launch_dp853_ens)(const PtRun *tab, int nmem, int nc, int minb, int block,
                                          int64_t ntot, cudaStream_t s)

@@ -23,9 +23,10 @@
  *     with cudaGetSymbolAddress (once per device, with that device current),
  *     and under CUDA's lazy module loading it is also the call that loads the
  *     library's kernels onto that device, which lets the driver allocate
- *     memory for them.  Make that first call at set-up time (np = 1 on a small
- *     grid will do) and before any stream capture; later calls allocate
- *     nothing;
+ *     memory for them: it launches those of both methods, for few particles
+ *     and for many, whatever it is asked to integrate.  Make that first call
+ *     at set-up time (np = 1 on a small grid will do) and before any stream
+ *     capture; later calls allocate nothing;
  *   - sharing: every call uses the same array and leaves its contents behind;
  *     each call re-packs the records it needs and zeroes the queue, flags and
  *     counter first.  Calls whose work overlaps on the GPU (other streams,
@@ -59,6 +60,7 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
 unsigned char *g_scratch_ptr[kMaxDevices] = {};
+bool g_ready[kMaxDevices] = {};
 
 /* Error text goes straight to the calling thread's pt_last_error buffer
  * (thread-local); messages are formatted on the caller's stack. */
@@ -90,6 +92,21 @@ int scratch_address(unsigned char **out, const char *who)
     }
     *out = g_scratch_ptr[dev];
     return PT_OK;
+}
+
+/* The first call on a device launches every kernel that a later call may need
+ * -- either method, few particles and many -- on no particles. */
+cudaError_t make_ready(const PtRun &R, cudaStream_t s)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(g_setup_mu);
+    if (g_ready[dev]) return cudaSuccess;
+    e = pt_ready_rk5(R, s);
+    if (e == cudaSuccess) e = pt_ready_dp853(R, s);
+    g_ready[dev] = e == cudaSuccess;
+    return e;
 }
 
 /* Planar reference layout -> node records {U, B}, written into the scratch. */
@@ -150,7 +167,12 @@ extern "C" int pt_integrate_device_noalloc(int32_t method, int64_t np, int32_t m
     if (rc != PT_OK) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     double *rec = reinterpret_cast<double *>(base + PT_NOALLOC_HEAD_BYTES);
-    cudaError_t e = cudaMemsetAsync(base, 0, PT_NOALLOC_HEAD_BYTES, s);
+    R.queue = reinterpret_cast<unsigned long long *>(base);
+    R.flags = reinterpret_cast<int32_t *>(base + sizeof(unsigned long long));
+    R.oob = reinterpret_cast<unsigned long long *>(base + 2 * sizeof(unsigned long long));
+    R.fresh = 1;
+    cudaError_t e = make_ready(R, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(base, 0, PT_NOALLOC_HEAD_BYTES, s);
     if (e == cudaSuccess && d_status) e = cudaMemsetAsync(d_status, 0xff, (size_t)np * sizeof(int32_t), s);
     if (e == cudaSuccess) {
         int64_t blocks = (nn + 255) / 256;
@@ -165,10 +187,6 @@ extern "C" int pt_integrate_device_noalloc(int32_t method, int64_t np, int32_t m
         R.cnt = d_cnt;
         R.status = d_status;
         R.carry = nullptr;
-        R.fresh = 1;
-        R.queue = reinterpret_cast<unsigned long long *>(base);
-        R.flags = reinterpret_cast<int32_t *>(base + sizeof(unsigned long long));
-        R.oob = reinterpret_cast<unsigned long long *>(base + 2 * sizeof(unsigned long long));
         R.nrec = nn;
         e = (method == PT_METHOD_RK5) ? pt_launch_rk5_exact(R, PT_NOALLOC_NC, s)
                                       : pt_launch_dp853_exact(R, PT_NOALLOC_NC, s);
