@@ -109,12 +109,14 @@ typedef struct pt_options {
                                      first (pt_run_device only), or NULL */
     int32_t       blocks_per_sm;  /* resident blocks per SM the kernel is compiled for:
                                      2, 3 or 4 (register caps 255, 168, 128); 0 = the
-                                     choice of pt_autotune for this kernel, else 3 */
+                                     choice of pt_autotune for this kernel, else 3; of
+                                     no effect on runs of at most 80 particles per SM */
     int32_t       interpolation;  /* 0: trilinear, interpolate_lin (interpolations.F90:104-226),
                                      the reference's choice; 1: the node at the lower
                                      corner of the cell, interpolate_near (:55-83) */
     int32_t       threads_per_block; /* 64, 128 or 256 (one particle per lane); 0 = the
-                                     choice of pt_autotune for this kernel, else 128 */
+                                     choice of pt_autotune for this kernel, else 128; as
+                                     blocks_per_sm, of no effect on small runs */
     double        open_x_margin;  /* with open_x: the escape faces sit this many domain
                                      lengths outside x = xmin and xmax (the field stays
                                      periodic); 0 = the domain faces */
@@ -183,13 +185,14 @@ int pt_run_device(int32_t method, int64_t np, int32_t m, const pt_fields *f,
  * PT_ERR_TIMEOUT or PT_ERR_CUDA. */
 int pt_run_check(const pt_fields *f);
 
-/* Launch autotuner: times the kernel that pt_run_device would launch with
- * these arguments in its launch variants and makes the fastest the default
- * (blocks_per_sm == 0, threads_per_block == 0) of that kernel family for the
- * rest of the process.  Search: the register cap of 2, 3 and 4 resident
- * 128-thread blocks per SM at 128 threads per block, then 64 and 256
- * threads per block at the best cap (one particle per lane throughout: the
- * lanes of a warp walk the stages in lock step).  The trial runs the first
+/* Launch autotuner: times the kernel that pt_run_device launches with these
+ * arguments for runs of more than 80 particles per SM (one lane per particle;
+ * smaller runs take eight, in a kernel without variants) in its launch
+ * variants and makes the fastest the default (blocks_per_sm == 0,
+ * threads_per_block == 0) of that kernel family for the rest of the process.
+ * Search: the register cap of 2, 3 and 4 resident 128-thread blocks per SM at
+ * 128 threads per block, then 64 and 256 threads per block at the best cap.
+ * The trial runs, on that kernel whatever their number, the first
  * `sample` particles (0: min(np, 2 x 4 x 128 per SM); < 0: all np) from
  * state(:,1,:) on scratch copies: up to opt->t_stop when it is > 0 -- a real
  * first window, outliers and tail included -- else max_steps attempts each

@@ -267,6 +267,7 @@ int prepare_run(int32_t method, int64_t np, int32_t m, const RunShape &g,
     R.budget_ns = (uint64_t)((budget > 0.0 ? budget : 600.0) * 1e9);
     R.m = m;
     R.np = np;
+    R.few = pt_coop_max();
     if (opt) {
         R.mlp = (opt->controller & PT_CTL_LEARNED)
                     ? pt_mlp_blob(static_cast<const pt_mlp *>(opt->model)) : nullptr;
@@ -333,7 +334,7 @@ void attach_fields(const pt_fields *f, PtRun &R)
 void attach_hand(const pt_fields *fc, PtRun &R)
 {
     pt_fields *f = const_cast<pt_fields *>(fc);
-    if (R.np <= pt_coop_max()) return;
+    if (R.np <= R.few) return;
     if (!f->hand) {
         /* In the default mode of a stream capture, here or in another thread, an
          * allocation invalidates the capture, be it of another stream than this
@@ -442,7 +443,10 @@ extern "C" int pt_autotune(int32_t method, int64_t np, int32_t m, const pt_field
     attach_fields(f, R);
     R.queue = f->scratch;
     R.flags = reinterpret_cast<int32_t *>(f->scratch + 1);
+    /* Variants are of the machine with one lane per particle, and the choice is for
+     * the runs that start on it: a smaller sample is timed there too, to its end. */
     attach_hand(f, R);
+    R.few = 0;
     if (!windowed && !(opt && opt->max_steps > 0)) R.max_steps = 32;
     /* One trial of variant (minb, block index) on fresh copies of the states. */
     auto trial = [&](int minb, int bi, bool keep) {

@@ -73,6 +73,7 @@ struct PtRun {
     /* sizes */
     int32_t m;
     int64_t np;
+    int64_t few;           /* a run of at most this many starts on eight lanes per particle */
     /* device pointers */
     const double *fld;     /* FP64 records */
     const float *fld32;    /* FP32 brick records (mixed precision) */

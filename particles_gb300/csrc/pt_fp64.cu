@@ -524,7 +524,7 @@ cudaError_t launch(const PtRun &P, cudaStream_t s)
 {
     if (P.np <= 0) return cudaSuccess;
     if (P.rec) return launch_v<METHOD, NC, true>(P, s);
-    const bool few = P.np <= pt_coop_max();
+    const bool few = P.np <= P.few;
     cudaError_t e = few ? cudaSuccess : P.mlp ? launch_v<METHOD, NC, true>(P, s) : launch_v<METHOD, NC, false>(P, s);
     if (e == cudaSuccess && (few || P.hand.ctl)) {
         if (P.mlp) e = pt_sm::launch_coop<METHOD, CoopF64<NC>>(k_coop<METHOD, NC, true>, few ? P.np : -1, true, s, P, few);

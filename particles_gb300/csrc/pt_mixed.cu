@@ -501,7 +501,7 @@ cudaError_t launch(const PtRun &P, cudaStream_t s)
     if (P.np <= 0) return cudaSuccess;
     if (LEARNABLE && P.rec) return launch_v<METHOD, EV, LEARNABLE>(P, s);
     const bool learn = LEARNABLE && P.mlp;
-    const bool few = P.np <= pt_coop_max();
+    const bool few = P.np <= P.few;
     cudaError_t e = few ? cudaSuccess : learn ? launch_v<METHOD, EV, LEARNABLE>(P, s) : launch_v<METHOD, EV, false>(P, s);
     if (e == cudaSuccess && (few || P.hand.ctl)) {
         if (learn) e = pt_sm::launch_coop<METHOD, EV>(k_coop_mixed<METHOD, EV, LEARNABLE>, few ? P.np : -1, true, s, P, few);
