@@ -407,6 +407,11 @@ int pt_debug_smul(int64_t n, const double *d_a, const double *d_b, double *d_out
  * the FP64 instructions they replace (4 doubles and 2 ints per input). */
 int pt_debug_intpipe(int64_t n, const double *d_x, int32_t d, double *d_out, int32_t *d_idx,
                      void *stream);
+/* The exact build's cell of one axis (interpolations.F90:140-149) of n positions
+ * d_x, in units of the domain, on d nodes: the offset d_xd[i] and the nodes
+ * d_lr[2i] and d_lr[2i + 1] left and right of it (device pointers). */
+int pt_debug_axis(int64_t n, const double *d_x, int32_t d, double *d_xd, int32_t *d_lr,
+                  void *stream);
 /* Constants of PT_CTL_FACE of one method for the runs prepared after the
  * call (all threads): faces within skip x the proposed step are crossed
  * (0 <= skip < 1; default 0.1 for RK5, 0.01 for DOP853) and steps end `over`

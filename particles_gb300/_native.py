@@ -34,7 +34,7 @@ EXPORTS = [
     "pt_ensemble_replay", "pt_ensemble_counts", "pt_ensemble_escaped", "pt_ensemble_check",
     "pt_copy_rows", "pt_debug_ctl_pow", "pt_debug_qdiv", "pt_debug_smul", "pt_last_transfer_bytes", "pt_debug_intpipe",
     "pt_initial_state", "pt_moments", "pt_debug_face_params", "pt_debug_face_cap",
-    "pt_debug_machines",
+    "pt_debug_machines", "pt_debug_axis",
 ]
 
 PT_INIT_SPEED, PT_INIT_GAMMA, PT_INIT_MAXWELLIAN = 0, 1, 2
@@ -126,6 +126,7 @@ def load():
     L.pt_debug_qdiv.argtypes = [i64, vp, vp, vp, vp]
     L.pt_debug_smul.argtypes = [i64, vp, vp, vp, vp]
     L.pt_debug_intpipe.argtypes = [i64, vp, i32, vp, vp, vp]
+    L.pt_debug_axis.argtypes = [i64, vp, i32, vp, vp, vp]
     L.pt_debug_accel.argtypes = [vp, i64, vp, vp, vp, vp]
     L.pt_probe_peak.argtypes = [i32, i32, C.POINTER(d)]
     L.pt_debug_unpack.argtypes = [i32, i64, i32, vp, i32, i32, vp, vp, vp]

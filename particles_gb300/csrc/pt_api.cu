@@ -638,6 +638,14 @@ extern "C" int pt_debug_intpipe(int64_t n, const double *d_x, int32_t d, double 
     return e == cudaSuccess ? PT_OK : cuda_err(e, "pt_debug_intpipe");
 }
 
+extern "C" int pt_debug_axis(int64_t n, const double *d_x, int32_t d, double *d_xd, int32_t *d_lr,
+                             void *stream)
+{
+    if (n < 0 || d < 1 || (n > 0 && (!d_x || !d_xd || !d_lr))) return set_err(PT_ERR_ARG, "bad argument%s");
+    const cudaError_t e = pt_launch_axis(n, d_x, d, d_xd, d_lr, (cudaStream_t)stream);
+    return e == cudaSuccess ? PT_OK : cuda_err(e, "pt_debug_axis");
+}
+
 extern "C" int pt_debug_qdiv(int64_t n, const double *d_a, const double *d_b, double *d_out,
                              void *stream)
 {

@@ -173,16 +173,15 @@ using PtR = double;
 #endif
 
 /* Fortran MIN/MAX with the NaN rule of the oracle (a NaN first operand
- * propagates), and maxval with NaN propagation. */
+ * propagates). */
 __device__ __forceinline__ double pt_max(double a, double b) { return (b > a) ? b : a; }
 __device__ __forceinline__ double pt_min(double a, double b) { return (b < a) ? b : a; }
-__device__ __forceinline__ double pt_nanmax(double m, double q) { return (q > m || q != q) ? q : m; }
 
 /* Comparisons on the integer pipe (an FP64 comparison takes an FP64 slot: with
  * them, the floors' hidden ones and the unused FP64 stage state gone, 262,144
  * particles RK5 FP32 25.6 -> 23.2 ms, DOP853 FP32 43.0 -> 39.8, RK5 exact
  * 57.5 -> 55.2).
- * pt_isnan for any x; pt_le: a <= b and pt_gt: a > b for b >= +0 and any a but NaN;
+ * pt_isnan for any x; pt_le: a <= b for b >= +0 and any a but NaN;
  * pt_max_pos: pt_max of magnitudes (a NaN may win where pt_max keeps a number). */
 __device__ __forceinline__ bool pt_isnan(double x)
 {
@@ -193,7 +192,6 @@ __device__ __forceinline__ bool pt_le(double a, double b)
 {
     return __double_as_longlong(a) <= __double_as_longlong(b);
 }
-__device__ __forceinline__ bool pt_gt(double a, double b) { return !pt_le(a, b); }
 __device__ __forceinline__ double pt_max_pos(double a, double b) { return pt_le(b, a) ? a : b; }
 
 /* floor(xp) as a 0-based node index; dm (only reachable when x - floor(x)
@@ -427,6 +425,8 @@ cudaError_t pt_launch_ctl_pow(int64_t n, const double *x, const double *y, doubl
                               cudaStream_t s);
 cudaError_t pt_launch_face_cap(const PtRun &P, int64_t n, const double *si, const double *h,
                                double *out, cudaStream_t s);
+cudaError_t pt_launch_axis(int64_t n, const double *x, int32_t d, double *xd, int32_t *lr,
+                           cudaStream_t s);
 cudaError_t pt_launch_intpipe(int64_t n, const double *x, int32_t d, double *out, int32_t *idx,
                               cudaStream_t s);
 

@@ -72,6 +72,16 @@ __global__ void k_smul(int64_t n, const double *a, const double *b, double *out)
     }
 }
 
+/* The exact build's cell of one axis: xd[i], lr[2i] and lr[2i + 1] of position x[i]
+ * on d nodes, the mask as a run sets it. */
+__global__ void k_axis(int64_t n, const double *x, int32_t d, double *xd, int32_t *lr)
+{
+    const double dmr = (double)d, inv_d = 1.0 / dmr;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        pt_axis_exact(x[i], d, (d & (d - 1)) == 0 ? d - 1 : 0, dmr, inv_d, lr[2 * i], lr[2 * i + 1], xd[i]);
+}
+
 /* The non-exact builds' controller power, for its accuracy test. */
 __global__ void k_ctl_pow(int64_t n, const double *x, const double *y, double *o)
 {
@@ -164,6 +174,15 @@ cudaError_t pt_launch_ctl_pow(int64_t n, const double *x, const double *y, doubl
     if (n <= 0) return cudaSuccess;
     const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
     k_ctl_pow<<<grid, 256, 0, s>>>(n, x, y, out);
+    return cudaGetLastError();
+}
+
+cudaError_t pt_launch_axis(int64_t n, const double *x, int32_t d, double *xd, int32_t *lr,
+                           cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
+    k_axis<<<grid, 256, 0, s>>>(n, x, d, xd, lr);
     return cudaGetLastError();
 }
 
