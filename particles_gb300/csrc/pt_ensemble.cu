@@ -39,7 +39,7 @@ struct pt_ensemble {
     PtRun *d_tab;
     double *d_tstop;
     int32_t *d_flags;
-    PtHand hand;                /* one allocation, ctl first */
+    PtHand hand;                /* ctl in d_flags; NULL where no window hands over */
     EnsBufs B;
     cudaGraph_t graph;
     cudaGraphExec_t exec;
@@ -75,7 +75,7 @@ __global__ void k_ens_init(EnsBufs B)
 /* Before a window: queue heads to 0, the queue length to the compacted one. */
 __global__ void k_ens_reset(EnsBufs B, unsigned long long *hand)
 {
-    if (threadIdx.x < 2) hand[threadIdx.x] = 0ull;
+    if (hand && threadIdx.x < 2) hand[threadIdx.x] = 0ull;
     const int k = threadIdx.x / PT_ENS_CTL, w = threadIdx.x % PT_ENS_CTL;
     if (k >= B.nmem) return;
     unsigned long long *c = B.ctl + (int64_t)k * PT_ENS_CTL;
@@ -234,7 +234,7 @@ static void ens_free(pt_ensemble *e)
     cudaFree(e->d_tab);
     cudaFree(e->d_tstop);
     cudaFree(e->d_flags);
-    cudaFree(e->hand.ctl);
+    cudaFree(e->hand.rec);
     cudaFree(e->B.ctl);
     cudaFree(e->B.idx);
     delete e;
@@ -284,7 +284,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
     }
     pt_ensemble *e = new pt_ensemble();
     memset(&e->B, 0, sizeof e->B);
-    e->hand.ctl = nullptr;
+    memset(&e->hand, 0, sizeof e->hand);
     e->method = method;
     e->precision = prec;
     e->nc = prec == PT_PREC_FP32 ? f0->nc32 : (prec == PT_PREC_BF16 ? f0->nc16 : f0->nc);
@@ -295,13 +295,25 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
     cudaGetDevice(&e->device);
     cudaError_t err = cudaMalloc(&e->d_tab, sizeof(PtRun) * nmembers);
     if (err == cudaSuccess) err = cudaMalloc(&e->d_tstop, sizeof(double));
-    if (err == cudaSuccess) err = cudaMalloc(&e->d_flags, 16);   /* flags, out-of-range count */
-    if (err == cudaSuccess) err = cudaMalloc(&e->hand.ctl, 256 + (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8);
+    if (err == cudaSuccess) err = cudaMalloc(&e->d_flags, 32);   /* flags, out-of-range count, hand.ctl */
     if (err == cudaSuccess) err = cudaMalloc(&e->B.ctl, sizeof(unsigned long long) * PT_ENS_CTL * nmembers);
     if (err == cudaSuccess) err = cudaMalloc(&e->B.idx, sizeof(int32_t) * (idx_elems > 0 ? idx_elems : 1));
     if (err != cudaSuccess) {
         ens_free(e);
         return set_err(PT_ERR_NOMEM, "ensemble buffers: %s", cudaGetErrorString(err));
+    }
+    /* The hand-over list, 5.8 MB (0.15 ms to create and destroy, 64 us without), is for
+     * ensembles whose windows may start on one lane per particle; without memory
+     * for it they keep their last particles there. */
+    if (ntot > pt_coop_max()) {
+        if (cudaMalloc(&e->hand.rec, (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8) == cudaSuccess) {
+            e->hand.ctl = reinterpret_cast<unsigned long long *>(e->d_flags + 4);
+            e->hand.lanes = pt_hand_lanes(ntot, prec);
+            e->hand.cap = pt_hand_cap();
+        } else {
+            e->hand.rec = nullptr;
+            (void)cudaGetLastError();
+        }
     }
     {   /* launch variant: as requested, else tuned for the single-run kernel, else default */
         PtRun probe = tab[0];
@@ -311,9 +323,6 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
         const int32_t tpb = pt_opt_threads_per_block(opt);
         e->block = tpb ? tpb : ((t >> 8) ? (t >> 8) : PT_BLOCK_DEFAULT);
     }
-    e->hand.rec = reinterpret_cast<double *>(e->hand.ctl + 32);
-    e->hand.lanes = pt_hand_lanes(ntot, prec);
-    e->hand.cap = pt_hand_cap();
     int64_t off = 0;
     for (int k = 0; k < nmembers; ++k) {
         const pt_member &M = members[k];

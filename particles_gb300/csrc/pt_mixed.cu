@@ -470,17 +470,19 @@ cudaError_t launch_ens(const PtRun *tab, int nmem, int minb, int block, int64_t 
 {
     if (ntot == 0) return cudaSuccess;          /* ntot < 0: configure only */
     if (!block) block = PT_BLOCK_DEFAULT;
-    cudaError_t e;
-    switch (minb) {
+    /* How many particles are left is known on the device only: both kernels are
+     * launched, and the one that is not to take the queue finds nothing.  An
+     * ensemble that never had more than `few` needs the second alone. */
+    const int64_t few = pt_coop_max();
+    cudaError_t e = cudaSuccess;
+    if (ntot < 0 || ntot > few) switch (minb) {
     case 2: e = launch_ens1<METHOD, EV, 2>(tab, nmem, block, ntot, s); break;
     case 4: e = launch_ens1<METHOD, EV, 4>(tab, nmem, block, ntot, s); break;
     default: e = launch_ens1<METHOD, EV, 3>(tab, nmem, block, ntot, s); break;
     }
-    /* how many particles are left is known on the device only: both kernels
-     * are launched, and the one that is not to take the queue finds nothing */
     if (e == cudaSuccess && ntot > 0)
-        e = pt_sm::launch_coop<METHOD, EV>(k_ensemble_coop_mixed<METHOD, EV>, -1, false, s, tab, nmem,
-                                           pt_coop_max());
+        e = pt_sm::launch_coop<METHOD, EV>(k_ensemble_coop_mixed<METHOD, EV>, ntot > few ? -1 : ntot, false, s, tab,
+                                            nmem, few);
     return e;
 }
 

@@ -71,3 +71,25 @@ def test_autotune_times_the_variants_on_a_small_sample(cuda):
     _, tried = f.autotune("dop853", prob["params"], b["time"], start, max_steps=32)
     print(min(ms), tried)
     assert min(tried.values()) > 1.6 * min(ms[1:])
+
+
+def test_a_small_ensemble_holds_no_hand_over_list(cuda):
+    """An ensemble that fits the eight-lane machine from its first window on never
+    hands particles over, so it does not pay for the list (5.8 MB, mapped and
+    unmapped with every ensemble)."""
+    torch = cuda
+    from particles_gb300 import Ensemble, Fields
+    prob = small_problem("rk5", n=12, npart=30, periods=0.05, seed=64, nsteps=2)
+    f = Fields(*prob["fields"])
+    z = lambda *shape, dtype: torch.zeros(shape, dtype=dtype, device="cuda")
+    member = dict(_buffers(torch, prob), fields=f, params=prob["params"], status=z(30, dtype=torch.int32),
+                  carry=z(128 * 30, dtype=torch.uint8))
+    Ensemble("rk5", [member]).close()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    held = Ensemble("rk5", [member])
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 2 << 20
+    held.run(0.0)
+    assert held.check() == 0 and held.counts()[0].sum() == 0
+    held.close()
