@@ -685,7 +685,8 @@ template <> struct Members<true> {
 };
 
 /* HAND: when the queue has run dry and at most PtHand.lanes lanes of a warp
- * still integrate, their particles go to the hand-over list. */
+ * still integrate, some of its particles having ended, theirs go to the
+ * hand-over list. */
 template <int METHOD, class EV, bool LEARN, bool ENS = false, bool HAND = false>
 __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
 {
@@ -942,12 +943,23 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                 const PtHand H = MB.q(0).hand;
                 if (H.ctl && !(LEARN && MB.q(0).rec)) {   /* recording keeps its pending records */
                     const int lane = threadIdx.x & 31;
+                    /* The last particles of a queue may be too few for a warp from the
+                     * start (np mod 32): handed over there, they would wait for the whole
+                     * launch to end.  So a warp waits until a particle of its own has
+                     * ended (L.n is 0 on lanes that never had one) or any other
+                     * warp has handed over.  13,000 particles of 16 attempts each, exact
+                     * RK5 1.57 -> 1.20 ms, DOP853 2.92 -> 2.25; FMA RK5 0.87 -> 0.67. */
+                    const bool ended = __any_sync(0xffffffffu, !active && L.n != 0);
                     unsigned long long at = 0;
-                    if (lane == 0)
-                        at = pt_hand_reserve(*(volatile unsigned long long *)H.ctl, __popc(act), H.cap,
-                                             [&](unsigned long long e, unsigned long long w) {
-                                                 return atomicCAS(H.ctl, e, w);
-                                             });
+                    if (lane == 0) {
+                        const unsigned long long seen = *(volatile unsigned long long *)H.ctl;
+                        at = ended || seen != 0ULL
+                                 ? pt_hand_reserve(seen, __popc(act), H.cap,
+                                                   [&](unsigned long long e, unsigned long long w) {
+                                                       return atomicCAS(H.ctl, e, w);
+                                                   })
+                                 : (unsigned long long)H.cap;
+                    }
                     at = __shfl_sync(0xffffffffu, at, 0);
                     if (at < (unsigned long long)H.cap) {
                         at += __popc(act & ((1u << lane) - 1u));

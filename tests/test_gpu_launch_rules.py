@@ -93,3 +93,31 @@ def test_a_small_ensemble_holds_no_hand_over_list(cuda):
     held.run(0.0)
     assert held.check() == 0 and held.counts()[0].sum() == 0
     held.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_the_last_particles_of_a_queue_start_with_the_others(cuda, native, precision):
+    """13,000 particles leave the last warp eight.  With the same number of attempts
+    each, a run in which warps may hand over takes as long as one in which they
+    may not (it took a third longer while that warp handed over at once)."""
+    torch = cuda
+    from particles_gb300 import Fields
+    prob = small_problem("rk5", n=16, npart=13000, periods=1.0, seed=65)
+    f, b = Fields(*prob["fields"], precision=precision), _buffers(torch, prob)
+    ms = {}
+    for cap in (0, -1):
+        native.pt_debug_machines(0, cap)
+        times = []
+        for _ in range(6):
+            b["state"].copy_(torch.tensor(prob["state"]))
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            f.run_device("rk5", prob["params"], b["time"], b["state"], b["cnt"], max_steps=16)
+            ev[1].record()
+            torch.cuda.synchronize()
+            times.append(ev[0].elapsed_time(ev[1]))
+        ms[cap] = min(times[1:])
+    native.pt_debug_machines(-1, -1)
+    print(ms)
+    assert (b["cnt"][:, 0] == 16).all()
+    assert ms[-1] < 1.12 * ms[0]
