@@ -105,8 +105,11 @@ __noinline__ __device__ float pt_pack_quotient(double v, float off, float sc)
  * v split into two floats, offset and 1/scale: within 7 FP32 ulps of the twice
  * rounded one, so their BF16 roundings agree unless a BF16 midpoint lies
  * within 8 ulps, and then (also where v nearly cancels the offset, or leaves
- * the FP32 normal range) the division decides.  256^3: 0.75 ms (0.45 without J);
- * with FP64 reductions and divisions it was 9.95 (6.91). */
+ * the FP32 normal range, as a zero does) the division decides.  256^3: 0.75 ms
+ * (0.45 without J); with FP64 reductions and divisions it was 9.95 (6.91).  With
+ * zeros the whole pt_fields_create_device call at 256^3 without J takes 0.62 ms
+ * (no component zero; 7.1 with FP64 reductions), 1.27 (Bz = 0; 7.6), 3.4 (U = 0;
+ * 8.6), 6.5 (all zero; 10.2). */
 template <int NV> struct PackShape {
     /* records per thread, blocks per SM; 1 x 2, 2 x 3, 3 x 3, 4 x 4 measured 944,
      * 748, 764, 868 us with J and 1 x 2, 2 x 3, 3 x 3, 3 x 4, 4 x 4 601, 535,
@@ -278,8 +281,15 @@ static int fields_create_impl(const int32_t dm[3], const double *uu, const doubl
 
     int rc = PT_OK;
     const size_t bytes3 = (size_t)dm[0] * dm[1] * dm[2] * 3 * sizeof(double);
-    /* host arrays that the packing kernels can read in place: no copies */
-    if (!on_device)
+    /* Host arrays that the packing kernels can read in place: no copies.  The BF16
+     * kernel reads a node up to eight times (1.42 times on average, in runs of 72
+     * bytes), which the link does not give back except on small grids.  In place /
+     * staged, pageable arrays without J: FP64 64^3 0.25 / 0.40 ms, 100^3 0.44 / 0.62,
+     * 256^3 4.4 / 5.5, 400^3 16.2 / 18.9; FP32 0.26 / 0.41, 0.51 / 0.62, 4.6 / 5.3, 16.7
+     * / 18.4; BF16 0.34 / 0.41, 0.74 / 0.65, 9.1 / 5.5, 34.4 / 19.4.  Pinned arrays and
+     * snapshots with J divide the same way. */
+    const bool in_place = precision != PT_PREC_BF16 || (int64_t)dm[0] * dm[1] * dm[2] <= 64 * 64 * 64;
+    if (!on_device && in_place)
         on_device = host_direct(uu, bytes3, false) && host_direct(bb, bytes3, false) &&
                     (!jj || host_direct(jj, bytes3, false));
     pt_fields *f = new pt_fields();
