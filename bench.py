@@ -1411,10 +1411,9 @@ def main():
         "data": "synthetic (seeded fields and particles)",
         "config": workload_config(cfg, npart, window, args),
         # a window is k_integrate and the k_coop that takes its last particles
-        # (a run of at most 80 particles per SM is k_coop alone)
+        # (k_coop alone for a run that starts on eight lanes per particle)
         "wall_s_timed": wall, "stopped_particles": stopped,
-        "gpu_launches": args.steps * (2 if npart > 80 * torch.cuda.get_device_properties(dev)
-                                      .multi_processor_count else 1),
+        "gpu_launches": args.steps * (2 if npart > L.pt_debug_machines(-1, -1) else 1),
         "rejected_fraction": float(dcnt_tot[2] / max(dcnt_tot[0], 1)),
         "attempts_per_s": float(dcnt_tot[0]) / elapsed,
         "particle_gyroperiods_per_s": world * npart * window * args.steps / elapsed,

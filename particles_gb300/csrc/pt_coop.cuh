@@ -5,7 +5,7 @@
  * What bounds such a run is not throughput but the time of one attempt: a
  * GB300 scheduler takes one FP64 warp instruction every 64 cycles, whatever
  * its active lanes and its independent work, so a particle advances at the
- * count of FP64 instructions its warp issues, ~2,500 per DOP853 attempt
+ * count of FP64 instructions its warp issues, ~2,400 per DOP853 attempt
  * (170 us) in the lane-per-particle machine of pt_integrator.cuh.  Here a
  * group of eight lanes shares them:
  *   - lane c < 6 owns component c of the state and its k rows: stage sums,

@@ -52,8 +52,10 @@
 
 /* Between the components of the DOP853 norm, exact build: keeps the compiler from
  * loading several components' k rows ahead, which spilled 430-500 bytes per thread
- * at 168 registers (now none at 150; 262,144 particles 61.1 -> 57.8 ms).  The
- * other builds do not spill there, and a fence would change what they contract. */
+ * at 168 registers (now none at 150; 262,144 particles 61.1 -> 57.8 ms).  With J and
+ * the learned controller 64 bytes are left (RK5: 124).  In the other builds a
+ * fence would change what is contracted; their DOP853 kernels do not spill there,
+ * but in ensembles, whose member table is indexed, by 178 to 378 bytes. */
 #ifdef PT_EXACT
 #define PT_FENCE asm volatile("" ::: "memory")
 #else
