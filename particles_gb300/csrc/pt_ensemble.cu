@@ -295,7 +295,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
     cudaGetDevice(&e->device);
     cudaError_t err = cudaMalloc(&e->d_tab, sizeof(PtRun) * nmembers);
     if (err == cudaSuccess) err = cudaMalloc(&e->d_tstop, sizeof(double));
-    if (err == cudaSuccess) err = cudaMalloc(&e->d_flags, 32);   /* flags, out-of-range count, hand.ctl */
+    if (err == cudaSuccess) err = cudaMalloc(&e->d_flags, 256);   /* flags, out-of-range count; at 128, hand.ctl */
     if (err == cudaSuccess) err = cudaMalloc(&e->B.ctl, sizeof(unsigned long long) * PT_ENS_CTL * nmembers);
     if (err == cudaSuccess) err = cudaMalloc(&e->B.idx, sizeof(int32_t) * (idx_elems > 0 ? idx_elems : 1));
     if (err != cudaSuccess) {
@@ -307,7 +307,7 @@ extern "C" int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_mem
      * for it they keep their last particles there. */
     if (ntot > pt_coop_max()) {
         if (cudaMalloc(&e->hand.rec, (size_t)PT_HAND_CAP * PT_HAND_WORDS * 8) == cudaSuccess) {
-            e->hand.ctl = reinterpret_cast<unsigned long long *>(e->d_flags + 4);
+            e->hand.ctl = reinterpret_cast<unsigned long long *>(e->d_flags + 32);
             e->hand.lanes = pt_hand_lanes(ntot, prec);
             e->hand.cap = pt_hand_cap();
         } else {
