@@ -360,7 +360,7 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
     if (LEARN) (void)pt_mlp_load(PT_Q.mlp, blob);
     uint64_t t_start = pt_globaltimer();
     const PtHand H = MB.q(0).hand;
-    const unsigned long long handed = H.ctl ? H.ctl[0] : 0ULL;
+    const unsigned long long handed = H.ctl ? pt_hand_written(H.ctl[0], H.cap) : 0ULL;
     Lane L;
     L.p = 0; L.t = 0.0; L.dt = 0.0; L.errold = 0.0; L.tnext = 0.0; L.n = 0;
     L.rejected = false; L.c0 = L.c1 = L.c2 = 0; L.w0 = 0;
@@ -409,10 +409,14 @@ __device__ __forceinline__ void run_coop(const Members<ENS> &MB, bool from_queue
                     if (handed && G.gl == 0) qi = atomicAdd(H.ctl + 1, 1ULL);
                     qi = G.get(qi, 0);
                     if (handed && qi < handed) {
-                        coop_take<METHOD>(H.rec + qi * PT_HAND_WORDS, G, K, L, si, t_start, mi);
-                        mode = M_READY;
-                        handed_over = true;
-                        active = true;
+                        const double *const r = H.rec + qi * PT_HAND_WORDS;
+                        /* (the next tail tries again after a slot marked as empty) */
+                        if (reinterpret_cast<const long long *>(r)[HandRec::P] >= 0) {
+                            coop_take<METHOD>(r, G, K, L, si, t_start, mi);
+                            mode = M_READY;
+                            handed_over = true;
+                            active = true;
+                        }
                     } else {
                         drained = true;
                     }

@@ -1,6 +1,15 @@
 /*
  * pt_hand.h -- slots of the hand-over list (PtHand), reserved by many warps at
  * once.  Host- and device-compilable; no dependencies.
+ *
+ * A warp with n particles adds n to the list's count, which nothing ever lowers,
+ * and has the n slots from the count before.  Where they do not all lie in the
+ * list it keeps its particles; if some do (one warp at most, the one that meets
+ * the end), it marks those as empty.  So every slot below the count and the
+ * list's end is written, by one warp each.  (Giving a range back where it does
+ * not fit leaves slots below the count that nobody writes; reserving by
+ * compare-and-swap makes some 1,800 warps that hand over together wait for one
+ * another: an ensemble's windows of 29 ms took 0.5 % longer.)
  */
 #ifndef PT_HAND_H
 #define PT_HAND_H
@@ -11,24 +20,19 @@
 #define PT_HAND_FN static inline
 #endif
 
-/* Reserves n consecutive slots of a list of cap: returns the first of them, or
- * cap if fewer than n are left.  cas(expected, wanted) compares and swaps the
- * list's count and returns what it held; seen is any value the count has held.
- * A reservation that does not fit leaves the count alone.  (Adding first and
- * subtracting when it did not fit lets another warp reserve above the sum in
- * between: the count then ends below slots that are written, and slots below
- * it are not.)  So the count never exceeds cap and every slot below it belongs
- * to exactly one reservation. */
-template <class CAS>
-PT_HAND_FN unsigned long long pt_hand_reserve(unsigned long long seen, unsigned long long n,
-                                              unsigned long long cap, CAS cas)
+/* Whether n slots from `at` on lie in a list of cap. */
+PT_HAND_FN bool pt_hand_fits(unsigned long long at, unsigned n, unsigned cap)
 {
-    while (n <= cap && seen <= cap - n) {
-        const unsigned long long was = cas(seen, seen + n);
-        if (was == seen) return seen;
-        seen = was;
-    }
-    return cap;
+    return at + n <= cap;
+}
+
+/* Whether slot i of a range that does not fit is in the list, to be marked. */
+PT_HAND_FN bool pt_hand_marks(unsigned long long i, unsigned cap) { return i < cap; }
+
+/* The slots written of a list of cap when its count is `count`. */
+PT_HAND_FN unsigned long long pt_hand_written(unsigned long long count, unsigned cap)
+{
+    return count < cap ? count : cap;
 }
 
 #endif /* PT_HAND_H */

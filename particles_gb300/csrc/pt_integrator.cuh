@@ -53,9 +53,9 @@
 /* Between the components of the DOP853 norm, exact build: keeps the compiler from
  * loading several components' k rows ahead, which spilled 430-500 bytes per thread
  * at 168 registers (now none at 150; 262,144 particles 61.1 -> 57.8 ms).  With J and
- * the learned controller 64 bytes are left (RK5: 124).  In the other builds a
+ * the learned controller 64 bytes are left (RK5: 132).  In the other builds a
  * fence would change what is contracted; their DOP853 kernels do not spill there,
- * but in ensembles, whose member table is indexed, by 178 to 378 bytes. */
+ * but in ensembles, whose member table is indexed, by 186 to 402 bytes. */
 #ifdef PT_EXACT
 #define PT_FENCE asm volatile("" ::: "memory")
 #else
@@ -952,22 +952,17 @@ __device__ __forceinline__ void run_machine(const Members<ENS> &MB)
                      * warp has handed over.  13,000 particles of 16 attempts each, exact
                      * RK5 1.57 -> 1.20 ms, DOP853 2.92 -> 2.25; FMA RK5 0.87 -> 0.67. */
                     const bool ended = __any_sync(0xffffffffu, !active && L.n != 0);
-                    unsigned long long at = 0;
-                    if (lane == 0) {
-                        const unsigned long long seen = *(volatile unsigned long long *)H.ctl;
-                        at = ended || seen != 0ULL
-                                 ? pt_hand_reserve(seen, __popc(act), H.cap,
-                                                   [&](unsigned long long e, unsigned long long w) {
-                                                       return atomicCAS(H.ctl, e, w);
-                                                   })
-                                 : (unsigned long long)H.cap;
-                    }
+                    unsigned long long at = (unsigned)H.cap;
+                    if (lane == 0 && (ended || *(volatile unsigned long long *)H.ctl != 0ULL))
+                        at = atomicAdd(H.ctl, (unsigned long long)__popc(act));
                     at = __shfl_sync(0xffffffffu, at, 0);
-                    if (at < (unsigned long long)H.cap) {
+                    if (pt_hand_fits(at, __popc(act), H.cap)) {
                         at += __popc(act & ((1u << lane) - 1u));
                         if (active) lane_hand<METHOD>(H.rec + at * PT_HAND_WORDS, K, L, si, t_start, mi);
                         break;
                     }
+                    if (lane < __popc(act) && pt_hand_marks(at + lane, H.cap))
+                        reinterpret_cast<long long *>(H.rec + (at + lane) * PT_HAND_WORDS)[HandRec::P] = -1;
                 }
             }
         }
