@@ -24,8 +24,8 @@
 
 /* Particles handed from the lane-per-particle machine to the eight-lane one
  * (pt_coop.cuh) when a launch runs out of queued particles: ctl[0] counts the
- * records (pt_hand.h), ctl[1] is the head they are taken from; a record holds a particle
- * between two attempts. */
+ * records (pt_hand.h), ctl[1] is the head they are taken from; a record holds a
+ * particle between two attempts. */
 #define PT_HAND_WORDS 22
 /* 16 warps on each of 152 SMs (the kernels' register counts allow no more) with
  * 12 particles each, or the warps of 240 particles per SM with 24 each; a warp
