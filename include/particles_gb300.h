@@ -250,11 +250,12 @@ int pt_ensemble_create(int32_t method, int32_t nmembers, const pt_member *member
 int pt_ensemble_destroy(pt_ensemble *e);
 
 /* One window: integrate every live particle of every member while
- * t < min(t_stop, tmax of its member) in ONE persistent launch, then compact
- * each member's work list -- particles that are done, escaped or failed
- * leave it; escaped ones are appended to the member's escaped list -- and
- * order it longest first by the attempts each particle needed in this
- * window.  Launches on `stream` without synchronising. */
+ * t < min(t_stop, tmax of its member) in ONE persistent launch (in ensembles of
+ * more than 80 particles per SM a second one takes what the first leaves at its
+ * end), then compact each member's work list -- particles that are done,
+ * escaped or failed leave it; escaped ones are appended to the member's
+ * escaped list -- and order it longest first by the attempts each particle
+ * needed in this window.  Launches on `stream` without synchronising. */
 int pt_ensemble_run(pt_ensemble *e, double t_stop, void *stream);
 
 /* Captures `windows` consecutive windows, each advancing the window end by
